@@ -13,11 +13,13 @@
 //
 // Antipodal batch: one thread per query (optionally in Hilbert order), the crossings by a
 // canonical traversal of the BVH4 with the stack in shared memory, the boundary term from
-// per-call edge records (both end points and the multiplicity, 32 bytes, read with warp-uniform
-// addresses) summed in FP64. Arithmetic is rounded operation by operation with dot products,
+// per-call row records (both end points and the multiplicity) summed in FP64: on the +z axis two rows
+// per packed instruction from a tile in shared memory, on the retried axes one by one. The crossings,
+// the singular tests and the retried axes are rounded operation by operation with dot products,
 // cross products and determinants fused in one fixed pattern that the oracle restates with fmaf;
 // the FP64 running sum replaces smallgwn's Kahan sum in float. Stack overflow writes NaN and sets
 // the BVH's device error bit instead of trapping.
+#include "gwnb_f32x2.cuh"
 #include "gwnb_internal.cuh"
 
 #include <algorithm>
@@ -218,13 +220,18 @@ template <int Axis> __device__ __forceinline__ bool triangle_crossing(v3 q, v3 a
     return true;
 }
 
+// Boundary rows in pairs, component by component: start xyz, end xyz and multiplicity of an even row,
+// each followed by the same of the odd one; the odd half of an unpaired last row repeats the even
+// one's ends with multiplicity 0.
+constexpr int k_row_pair = 16;
+
 struct antipodal_params {
     float4 const *nodes; // node_count x 8 float4
     std::uint64_t node_count;
     triangle48 const *tri48;
     std::uint64_t primitive_count;
     std::uint64_t root_ref;
-    float4 const *edges; // 2 float4 per boundary row: (start, multiplicity), (end, 0)
+    float const *edges; // boundary rows in pairs (k_row_pair floats each, see load_row)
     std::uint64_t edge_count;
     float const *qx, *qy, *qz;
     std::uint32_t const *order;
@@ -368,6 +375,13 @@ template <int Axis> __device__ __forceinline__ area_args_d area_arguments_d(floa
     return r;
 }
 
+// Boundary row i as (start, multiplicity) and (end, 0).
+__device__ __forceinline__ void load_row(float const *edges, std::uint64_t i, float4 &A, float4 &B) {
+    float const *r = edges + (i >> 1) * k_row_pair + (i & 1u);
+    A = make_float4(__ldg(r), __ldg(r + 2), __ldg(r + 4), __ldg(r + 12));
+    B = make_float4(__ldg(r + 6), __ldg(r + 8), __ldg(r + 10), 0.0f);
+}
+
 // One boundary row against query q: the end points relative to q.
 __device__ __forceinline__ void row_ends(float4 A, float4 B, v3 q, v3 &s, v3 &e) {
     s = {__fsub_rn(A.x, q.x), __fsub_rn(A.y, q.y), __fsub_rn(A.z, q.z)};
@@ -406,7 +420,9 @@ template <int Axis> __device__ __forceinline__ bool boundary_term(antipodal_para
     double sum = 0.0;
     for (std::uint64_t i = 0; i < p.edge_count; ++i) {
         double term;
-        if (!row_term<Axis>(__ldg(p.edges + 2 * i), __ldg(p.edges + 2 * i + 1), q, term))
+        float4 A, B;
+        load_row(p.edges, i, A, B);
+        if (!row_term<Axis>(A, B, q, term))
             return false;
         sum += term;
     }
@@ -428,81 +444,166 @@ template <int Axis> __device__ __forceinline__ int antipodal_axis(antipodal_para
     return 0;
 }
 
-// Value batch (:533-568): k_ap_q queries per thread. The +z axis, which decides almost every query,
-// runs for the whole block together: crossings per thread, then the boundary rows in tiles of
-// k_ap_tile staged in shared memory and shared by all queries of the block. A query whose +z
-// crossings or boundary rows are singular retries +x and +y on its own (global loads). One query
-// per thread fits 60 registers (4 resident blocks of 256) where two took 80 (3 blocks): 11 % less
-// time on 1M queries against 2,048 boundary rows, results bit-identical.
-constexpr int k_ap_tile = 256;
-constexpr int k_ap_q = 1;
+// ---- boundary rows in pairs, +z axis ----------------------------------------------------------------
+//
+// The +z axis decides almost every query, so its rows run packed, two per instruction, without the
+// guarded branch of row_term: on an open soup 2.5 % of the (row, query) pairs pass close enough to the
+// ray line to be guarded, some lane of a warp in 36 % of the rows, and the FP64 of that branch was most
+// of the time. The arguments are formed so that they do not cancel there. With unit vectors s, e,
+// 1 - s_z - e_z + s.e = (1 - s_z)(1 - e_z) + s_xy . e_xy, and 1 - s_z = |s_xy|^2 / (1 + s_z) on the side
+// where it cancels; an end point is kept as a positive multiple of (s_xy, 1 - s_z):
+//   s_z > 0: ((1 + |s_z|) s_xy, |s_xy|^2),   s_z <= 0: (s_xy, 1 + |s_z|),
+// and num, den are -det and dot product of such vectors. s_xy = V_xy - q_xy is exact to its last bit,
+// so are det and the dot product in relation to |s_xy||e_xy|, and what is left of den's rounding is
+// that of well conditioned products. What remains ill conditioned is a row whose end points lie on
+// opposite sides of the query (s.e near -|s||e|: the query almost on the edge); those take row_term.
+// Bound by the FP32 pipe (27 packed operations per row) and the special-function unit (two square
+// roots, a reciprocal and a conversion per row). 200,000 queries against 7,406 rows, value and
+// gradient: 29.4 ms row by row, 7.7 ms in pairs; against FP64 the value's error falls from 4.1e-7 to
+// 2.9e-7 (2-norm) and the gradient's from 3e-7 to 4e-8.
 
+constexpr int k_ap_tile = 256;                  // rows per tile
+constexpr float k_ap_opposed = 1.0f / 64.0f;    // 1 + cos(s, e) below which a row takes its FP64 form
+
+// One half of a pair, after the packed part: the residual angle r (|r| <= pi/4) carries the signs of the
+// quadrant and quarters the rest, so that angle = r + quarters pi/2.
+__device__ __forceinline__ void quadrant(float num, float den, float &r, float &quarters) {
+    bool const swap = fabsf(num) > fabsf(den);
+    unsigned const sn = __float_as_uint(num) & 0x80000000u, sd = __float_as_uint(den) & 0x80000000u;
+    float const k = swap ? 1.0f : (sd != 0u ? 2.0f : 0.0f);
+    quarters = __uint_as_float(__float_as_uint(k) | sn);
+    r = __uint_as_float(__float_as_uint(r) ^ sn ^ sd ^ (swap ? 0x80000000u : 0u));
+}
+
+// An end point's scale and height (see above) from z / |v| and |v_xy|^2 / |v|^2.
+__device__ __forceinline__ void end_form(float z, float u, float &g, float &h) {
+    float const m = 1.0f + fabsf(z);
+    bool const up = z > 0.0f;
+    g = up ? m : 1.0f;
+    h = up ? u : m;
+}
+
+struct row_pair {
+    x2::f2 sx, sy, sz, ex, ey, ez, m;
+};
+__device__ __forceinline__ row_pair load_row_pair(float const *p) {
+    ulonglong2 const *w = reinterpret_cast<ulonglong2 const *>(p);
+    ulonglong2 const a = w[0], b = w[1], c = w[2], d = w[3];
+    return row_pair{{a.x}, {a.y}, {b.x}, {b.y}, {c.x}, {c.y}, {d.x}};
+}
+
+// Singular on +z (classify): a collinear projection whose ends lie on opposite sides of the query.
+__device__ __forceinline__ bool row_singular(float det, float c0) { return det == 0.0f && c0 <= 0.0f; }
+
+// A pair's angles: residuals times multiplicity added to sum, quarters times multiplicity to quarters.
+// True when a half is singular or opposed: nothing is added and the caller takes the rows one by one.
+__device__ __forceinline__ bool area_pair(row_pair const &t, x2::f2 nqx, x2::f2 nqy, x2::f2 nqz, double &sum,
+                                          float &quarters) {
+    using namespace x2;
+    f2 const sx = add(t.sx, nqx), sy = add(t.sy, nqy), sz = add(t.sz, nqz);
+    f2 const ex = add(t.ex, nqx), ey = add(t.ey, nqy), ez = add(t.ez, nqz);
+    f2 const ps = fma(sy, sy, mul(sx, sx)), pe = fma(ey, ey, mul(ex, ex));
+    f2 const rs = rsqrt_newton(fma(sz, sz, ps)), re = rsqrt_newton(fma(ez, ez, pe));
+    // the projected determinant in classify's rounding pattern, and the projected dot product
+    f2 const det = fma(sx, ey, mul(mul(sy, ex), both(-1.0f)));
+    f2 const c0 = fma(sy, ey, mul(sx, ex));
+    f2 const rr = mul(rs, re);
+    float d0, d1, o0, o1;
+    unpack(det, d0, d1);
+    unpack(fma(fma(sz, ez, c0), rr, both(1.0f)), o0, o1);
+    if (fminf(fabsf(d0), fabsf(d1)) == 0.0f || fminf(o0, o1) < k_ap_opposed)
+        return true;
+    f2 const us = mul(mul(ps, rs), rs), ue = mul(mul(pe, re), re);
+    float z0, z1, u0, u1, gs0, gs1, hs0, hs1, ge0, ge1, he0, he1;
+    unpack(mul(sz, rs), z0, z1);
+    unpack(us, u0, u1);
+    end_form(z0, u0, gs0, hs0);
+    end_form(z1, u1, gs1, hs1);
+    unpack(mul(ez, re), z0, z1);
+    unpack(ue, u0, u1);
+    end_form(z0, u0, ge0, he0);
+    end_form(z1, u1, ge1, he1);
+    f2 const kk = mul(rr, mul(pack(gs0, gs1), pack(ge0, ge1)));
+    f2 const num = mul(det, mul(kk, both(-1.0f)));
+    f2 const den = fma(c0, kk, mul(pack(hs0, hs1), pack(he0, he1)));
+    float n0, n1, e0, e1, r0, r1, k0, k1, m0, m1;
+    unpack(num, n0, n1);
+    unpack(den, e0, e1);
+    f2 const lo = pack(fminf(fabsf(n0), fabsf(e0)), fminf(fabsf(n1), fabsf(e1)));
+    f2 const hi = pack(fmaxf(fabsf(n0), fabsf(e0)), fmaxf(fabsf(n1), fabsf(e1)));
+    unpack(mul(atan_one(divide(lo, hi)), t.m), r0, r1);
+    unpack(t.m, m0, m1);
+    quadrant(n0, e0, r0, k0);
+    quadrant(n1, e1, r1, k1);
+    sum += static_cast<double>(r0);
+    sum += static_cast<double>(r1);
+    quarters = __fmaf_rn(k1, m1, __fmaf_rn(k0, m0, quarters));
+    return false;
+}
+
+// Value batch (:533-568), one query per thread: crossings per thread, then the boundary rows in tiles
+// of k_ap_tile staged in shared memory and shared by all queries of the block. A query whose +z
+// crossings or boundary rows are singular retries +x and +y on its own (global loads), and one whose
+// packed sum is not a number (end points too close or too far for the approximate reciprocals, or not
+// numbers themselves) sums its +z rows again one by one.
 __global__ void __launch_bounds__(256) k_antipodal(antipodal_params p) {
-    extern __shared__ float4 s_dyn[]; // [2 * k_ap_tile] edge tile, then [p.stack_cap][blockDim.x] stack
-    float4 *s_rows = s_dyn;
-    std::uint32_t *s_stack = reinterpret_cast<std::uint32_t *>(s_dyn + 2 * k_ap_tile) + threadIdx.x;
-    std::uint64_t const base_idx = static_cast<std::uint64_t>(blockIdx.x) * blockDim.x * k_ap_q + threadIdx.x;
-    std::uint32_t qi[k_ap_q];
-    v3 q[k_ap_q];
-    float cross[k_ap_q];
-    int rc[k_ap_q]; // 0 done so far, 1 singular on +z, 2 overflow, 3 no query
-    double sum[k_ap_q];
-#pragma unroll
-    for (int k = 0; k < k_ap_q; ++k) {
-        std::uint64_t const idx = base_idx + static_cast<std::uint64_t>(k) * blockDim.x;
-        sum[k] = 0.0;
-        cross[k] = 0.0f;
-        if (idx >= p.n) {
-            rc[k] = 3;
-            qi[k] = 0;
-            q[k] = {0.0f, 0.0f, 0.0f};
-            continue;
-        }
-        qi[k] = p.order != nullptr ? p.order[idx] : static_cast<std::uint32_t>(idx);
-        q[k] = {p.qx[qi[k]], p.qy[qi[k]], p.qz[qi[k]]};
-        rc[k] = crossings<2>(p, q[k], s_stack, cross[k]);
-    }
+    extern __shared__ float4 s_dyn[]; // row tile, then [p.stack_cap][blockDim.x] stack
+    float *s_rows = reinterpret_cast<float *>(s_dyn);
+    std::uint32_t *s_stack = reinterpret_cast<std::uint32_t *>(s_dyn + k_ap_tile / 2 * k_row_pair / 4) + threadIdx.x;
+    std::uint64_t const idx = static_cast<std::uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    bool const valid = idx < p.n;
+    std::uint32_t const qi = valid ? (p.order != nullptr ? p.order[idx] : static_cast<std::uint32_t>(idx)) : 0u;
+    v3 const q = valid ? v3{p.qx[qi], p.qy[qi], p.qz[qi]} : v3{0.0f, 0.0f, 0.0f};
+    float cross = 0.0f;
+    int rc = valid ? crossings<2>(p, q, s_stack, cross) : 3; // 0 done so far, 1 singular on +z, 2 overflow, 3 no query
+    x2::f2 const nqx = x2::both(-q.x), nqy = x2::both(-q.y), nqz = x2::both(-q.z);
+    double sum = 0.0;  // residual angles (half areas)
+    double turns = 0.0; // quarter turns
     for (std::uint64_t base = 0; base < p.edge_count; base += k_ap_tile) {
         int const cnt = static_cast<int>(p.edge_count - base < k_ap_tile ? p.edge_count - base : k_ap_tile);
+        int const pairs = (cnt + 1) / 2;
         __syncthreads();
-        for (int t = threadIdx.x; t < 2 * cnt; t += blockDim.x)
-            s_rows[t] = __ldg(p.edges + 2 * base + t);
+        for (int t = threadIdx.x; t < pairs * (k_row_pair / 4); t += blockDim.x)
+            s_dyn[t] = __ldg(reinterpret_cast<float4 const *>(p.edges + base / 2 * k_row_pair) + t);
         __syncthreads();
-        // four rows in flight: their square roots and atan2 interleave (the FP64 sum still adds
-        // the terms in row order); 2-4 % less time, results bit-identical
-#pragma unroll 4
-        for (int j = 0; j < cnt; ++j) {
-            float4 const A = s_rows[2 * j], B = s_rows[2 * j + 1];
-#pragma unroll
-            for (int k = 0; k < k_ap_q; ++k) {
-                if (rc[k] != 0)
-                    continue;
+        float quarters = 0.0f;
+        for (int j = 0; j < pairs; ++j) {
+            if (!area_pair(load_row_pair(s_rows + j * k_row_pair), nqx, nqy, nqz, sum, quarters))
+                continue;
+            for (int h = 0; h < 2 && rc == 0; ++h) {
+                std::uint64_t const i = base + static_cast<std::uint64_t>(2 * j + h);
+                if (i >= p.edge_count)
+                    break;
+                float4 A, B;
+                load_row(p.edges, i, A, B);
                 double term;
-                if (row_term<2>(A, B, q[k], term))
-                    sum[k] += term;
+                if (row_term<2>(A, B, q, term))
+                    sum += 0.5 * term;
                 else
-                    rc[k] = 1;
+                    rc = 1;
             }
         }
+        turns += static_cast<double>(quarters);
     }
-#pragma unroll
-    for (int k = 0; k < k_ap_q; ++k) {
-        if (rc[k] == 3)
-            continue;
-        float result = __int_as_float(0x7fc00000);
-        int r = rc[k];
-        if (r == 0)
-            result = static_cast<float>(static_cast<double>(cross[k]) + sum[k] / (4.0 * k_pi_d));
-        if (r == 1)
-            r = antipodal_axis<0>(p, q[k], s_stack, result);
-        if (r == 1)
-            r = antipodal_axis<1>(p, q[k], s_stack, result);
-        if (r == 2)
-            atomicOr(p.status, k_err_stack_overflow);
-        if (r != 0)
-            result = __int_as_float(0x7fc00000);
-        p.out[qi[k]] = result;
+    if (rc == 3)
+        return;
+    float result = __int_as_float(0x7fc00000);
+    if (rc == 0) {
+        double b = (2.0 * sum + turns * k_pi_d) / (4.0 * k_pi_d);
+        if (isnan(b) && !boundary_term<2>(p, q, b))
+            rc = 1;
+        else
+            result = static_cast<float>(static_cast<double>(cross) + b);
     }
+    if (rc == 1)
+        rc = antipodal_axis<0>(p, q, s_stack, result);
+    if (rc == 1)
+        rc = antipodal_axis<1>(p, q, s_stack, result);
+    if (rc == 2)
+        atomicOr(p.status, k_err_stack_overflow);
+    if (rc != 0)
+        result = __int_as_float(0x7fc00000);
+    p.out[qi] = result;
 }
 
 // :261-304: gradient of one signed spherical-area term with respect to the query (float).
@@ -582,7 +683,9 @@ template <int Axis> __device__ __forceinline__ bool boundary_gradient(antipodal_
     double sx = 0.0, sy = 0.0, sz = 0.0;
     for (std::uint64_t i = 0; i < p.edge_count; ++i) {
         double t[3];
-        if (!row_gradient<Axis>(__ldg(p.edges + 2 * i), __ldg(p.edges + 2 * i + 1), q, t))
+        float4 A, B;
+        load_row(p.edges, i, A, B);
+        if (!row_gradient<Axis>(A, B, q, t))
             return false;
         sx += t[0];
         sy += t[1];
@@ -593,29 +696,120 @@ template <int Axis> __device__ __forceinline__ bool boundary_gradient(antipodal_
     return true;
 }
 
-// Gradient batch (:336-372), tiled like the value batch on the +z axis, one query per thread.
+// Gradient batch (:336-372), tiled like the value batch on the +z axis, one query per thread. A row's
+// term is the gradient of the area of (-ray, s, e): the line integral of (x - q) x dx / |x - q|^3 along
+// the edge plus that along the two half lines from its ends in direction -ray. A boundary chain is
+// closed -- every vertex starts as many of its rows as it ends, with multiplicity -- so the half
+// lines cancel between rows and only the edges' integrals are summed:
+//   (s x e) (1/|s| + 1/|e|) / (|s||e| + s.e),   s x e = s x (e - s),
+// which does not grow where the edge passes the ray line, so no row needs the FP64 of row_gradient
+// there (half of the time of a batch went to those and to the four divisions of a row). A row whose
+// ends lie on opposite sides of the query takes its FP64 form; a query with a singular row retries
+// +x and +y with the areas' own gradients, and one whose sum is not a number sums its +z rows that way.
+constexpr float k_grad_opposed = 0.5f; // 1 + cos(s, e) below which a row's term is formed in FP64: the edges
+                                       // nearest to a query, whose terms are the largest
+constexpr int k_grad_pair = 28;        // a pair's 14 floats, then e - s and s - e
+
+struct grad_pair {
+    row_pair r;
+    x2::f2 lx, ly, lz, mx, my, mz; // e - s and s - e
+};
+__device__ __forceinline__ grad_pair load_grad_pair(float const *p) {
+    ulonglong2 const *w = reinterpret_cast<ulonglong2 const *>(p);
+    ulonglong2 const a = w[0], b = w[1], c = w[2], d = w[3], e = w[4], f = w[5], g = w[6];
+    return grad_pair{{{a.x}, {a.y}, {b.x}, {b.y}, {c.x}, {c.y}, {d.x}}, {d.y}, {e.x}, {e.y}, {f.x}, {f.y}, {g.x}};
+}
+
+// The edge's integral in FP64 from the float end points and query, times the multiplicity.
+__device__ __forceinline__ void edge_gradient_d(float4 A, float4 B, v3 q, double g[3]) {
+    double const s[3] = {static_cast<double>(A.x) - q.x, static_cast<double>(A.y) - q.y, static_cast<double>(A.z) - q.z};
+    double const e[3] = {static_cast<double>(B.x) - q.x, static_cast<double>(B.y) - q.y, static_cast<double>(B.z) - q.z};
+    double const c[3] = {s[1] * e[2] - s[2] * e[1], s[2] * e[0] - s[0] * e[2], s[0] * e[1] - s[1] * e[0]};
+    double const ls = sqrt(s[0] * s[0] + s[1] * s[1] + s[2] * s[2]);
+    double const le = sqrt(e[0] * e[0] + e[1] * e[1] + e[2] * e[2]);
+    double const dt = s[0] * e[0] + s[1] * e[1] + s[2] * e[2], pr = ls * le;
+    // |s||e| + s.e = |s x e|^2 / (|s||e| - s.e) where it cancels
+    double const sm = dt < 0.0 ? (c[0] * c[0] + c[1] * c[1] + c[2] * c[2]) / (pr - dt) : pr + dt;
+    double const f = static_cast<double>(A.w) * (ls + le) / (pr * sm);
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        g[k] = f * c[k];
+}
+
+// True when a half is singular or opposed (see area_pair).
+__device__ __forceinline__ bool gradient_pair(grad_pair const &t, x2::f2 nqx, x2::f2 nqy, x2::f2 nqz, double (&g)[3]) {
+    using namespace x2;
+    f2 const sx = add(t.r.sx, nqx), sy = add(t.r.sy, nqy), sz = add(t.r.sz, nqz);
+    f2 const ex = add(t.r.ex, nqx), ey = add(t.r.ey, nqy), ez = add(t.r.ez, nqz);
+    f2 const rs = rsqrt_newton(dot(sx, sy, sz, sx, sy, sz)), re = rsqrt_newton(dot(ex, ey, ez, ex, ey, ez));
+    f2 const det = fma(sx, ey, mul(mul(sy, ex), both(-1.0f)));
+    f2 const rr = mul(rs, re);
+    float d0, d1, o0, o1;
+    unpack(det, d0, d1);
+    f2 const o = fma(dot(sx, sy, sz, ex, ey, ez), rr, both(1.0f));
+    unpack(o, o0, o1);
+    if (fminf(fabsf(d0), fabsf(d1)) == 0.0f || fminf(o0, o1) < k_grad_opposed)
+        return true;
+    f2 const f = divide(mul(mul(add(rs, re), rr), t.r.m), o);
+    f2 const c[3] = {mul(fma(sy, t.lz, mul(sz, t.my)), f), mul(fma(sz, t.lx, mul(sx, t.mz)), f),
+                     mul(fma(sx, t.ly, mul(sy, t.mx)), f)};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        float a, b;
+        unpack(c[k], a, b);
+        g[k] += static_cast<double>(a);
+        g[k] += static_cast<double>(b);
+    }
+    return false;
+}
+
 __global__ void __launch_bounds__(256) k_antipodal_gradient(antipodal_params p) {
-    __shared__ float4 s_rows[2 * k_ap_tile];
+    __shared__ __align__(16) float s_rows[k_ap_tile / 2 * k_grad_pair];
     std::uint64_t const idx = static_cast<std::uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     bool const valid = idx < p.n;
     std::uint32_t const qi = valid ? (p.order != nullptr ? p.order[idx] : static_cast<std::uint32_t>(idx)) : 0u;
     v3 const q = valid ? v3{p.qx[qi], p.qy[qi], p.qz[qi]} : v3{0.0f, 0.0f, 0.0f};
+    x2::f2 const nqx = x2::both(-q.x), nqy = x2::both(-q.y), nqz = x2::both(-q.z);
     bool ok = valid;
-    double sx = 0.0, sy = 0.0, sz = 0.0;
+    double sum[3] = {0.0, 0.0, 0.0};
     for (std::uint64_t base = 0; base < p.edge_count; base += k_ap_tile) {
         int const cnt = static_cast<int>(p.edge_count - base < k_ap_tile ? p.edge_count - base : k_ap_tile);
+        int const pairs = (cnt + 1) / 2;
         __syncthreads();
-        for (int t = threadIdx.x; t < 2 * cnt; t += blockDim.x)
-            s_rows[t] = __ldg(p.edges + 2 * base + t);
+        for (int t = threadIdx.x; t < 2 * pairs; t += blockDim.x) {
+            float const *r = p.edges + (base + t) / 2 * k_row_pair + (t & 1);
+            float *w = s_rows + t / 2 * k_grad_pair + (t & 1);
+#pragma unroll
+            for (int k = 0; k < 7; ++k)
+                w[2 * k] = __ldg(r + 2 * k);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                float const l = w[2 * k + 6] - w[2 * k];
+                w[2 * k + 14] = l;
+                w[2 * k + 20] = -l;
+            }
+        }
         __syncthreads();
-        for (int j = 0; j < cnt && ok; ++j) {
-            double t[3];
-            if (row_gradient<2>(s_rows[2 * j], s_rows[2 * j + 1], q, t)) {
-                sx += t[0];
-                sy += t[1];
-                sz += t[2];
-            } else {
-                ok = false;
+        for (int j = 0; j < pairs; ++j) {
+            if (!gradient_pair(load_grad_pair(s_rows + j * k_grad_pair), nqx, nqy, nqz, sum))
+                continue;
+            for (int h = 0; h < 2 && ok; ++h) {
+                std::uint64_t const i = base + static_cast<std::uint64_t>(2 * j + h);
+                if (i >= p.edge_count)
+                    break;
+                float4 A, B;
+                load_row(p.edges, i, A, B);
+                v3 s, e;
+                row_ends(A, B, q, s, e);
+                if (classify<2>(s, e).singular) {
+                    ok = false;
+                } else {
+                    double g[3];
+                    edge_gradient_d(A, B, q, g);
+#pragma unroll
+                    for (int k = 0; k < 3; ++k)
+                        sum[k] += g[k];
+                }
             }
         }
     }
@@ -624,28 +818,33 @@ __global__ void __launch_bounds__(256) k_antipodal_gradient(antipodal_params p) 
     float const nan = __int_as_float(0x7fc00000);
     v3 g{nan, nan, nan};
     double const k4 = 4.0 * k_pi_d;
-    if (ok)
-        g = {static_cast<float>(sx / k4), static_cast<float>(sy / k4), static_cast<float>(sz / k4)};
-    else if (!boundary_gradient<0>(p, q, g) && !boundary_gradient<1>(p, q, g))
+    if (ok && !isnan(sum[0] + sum[1] + sum[2]))
+        g = {static_cast<float>(sum[0] / k4), static_cast<float>(sum[1] / k4), static_cast<float>(sum[2] / k4)};
+    else if (!(ok && boundary_gradient<2>(p, q, g)) && !boundary_gradient<0>(p, q, g) && !boundary_gradient<1>(p, q, g))
         g = {nan, nan, nan};
     p.gx[qi] = g.x;
     p.gy[qi] = g.y;
     p.gz[qi] = g.z;
 }
 
-// Edge records of the chain over the current positions: (start, multiplicity), (end, 0).
+// Row records of the chain over the current positions (see k_row_pair).
 __global__ void __launch_bounds__(256)
     k_edge_records(gwnb_geometry_f32 g, std::uint32_t const *__restrict__ start, std::uint32_t const *__restrict__ end,
-                   std::uint64_t const *__restrict__ mult, std::uint64_t n, float4 *__restrict__ out) {
+                   std::uint64_t const *__restrict__ mult, std::uint64_t n, float *__restrict__ out) {
     std::uint64_t const i = static_cast<std::uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n)
+    if (i >= (n + 1) / 2 * 2)
         return;
-    std::uint32_t const a = start[i], b = end[i];
+    std::uint64_t const row = i < n ? i : n - 1;
+    std::uint32_t const a = start[row], b = end[row];
     bool const ok = a < g.vertex_count && b < g.vertex_count;
     float const nan = __int_as_float(0x7fc00000);
-    out[2 * i] = ok ? make_float4(g.vertex_x[a], g.vertex_y[a], g.vertex_z[a], static_cast<float>(mult[i]))
-                    : make_float4(nan, nan, nan, 0.0f);
-    out[2 * i + 1] = ok ? make_float4(g.vertex_x[b], g.vertex_y[b], g.vertex_z[b], 0.0f) : make_float4(nan, nan, nan, 0.0f);
+    float const v[8] = {ok ? g.vertex_x[a] : nan, ok ? g.vertex_y[a] : nan, ok ? g.vertex_z[a] : nan,
+                        ok ? g.vertex_x[b] : nan, ok ? g.vertex_y[b] : nan, ok ? g.vertex_z[b] : nan,
+                        ok && i < n ? static_cast<float>(mult[row]) : 0.0f, 0.0f};
+    float *o = out + i / 2 * k_row_pair + (i & 1u);
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        o[2 * k] = v[k];
 }
 
 int bits_for(std::uint64_t v) {
@@ -804,7 +1003,7 @@ static int antipodal_common(const gwnb_geometry_f32 *g, const gwnb_bvh4_f32 *b_i
             return set_error(GWNB_INVALID_ARGUMENT, "Traversal stack capacity is below the BVH internal stack bound.");
         if (ref_internal(b_in->root.reference) &&
             static_cast<std::uint64_t>(b_in->internal_stack_bound) * query_launch_block(o.block_size) * 4u +
-                    2u * k_ap_tile * 16u >
+                    k_ap_tile / 2 * k_row_pair * sizeof(float) >
                 227u * 1024u)
             return set_error(GWNB_INVALID_ARGUMENT,
                              "Traversal stack bound times block size exceeds the 227 KB of shared memory per block.");
@@ -840,12 +1039,13 @@ static int antipodal_common(const gwnb_geometry_f32 *g, const gwnb_bvh4_f32 *b_i
         if (p.stack_cap < 1)
             p.stack_cap = 1;
     }
-    float4 *edges = nullptr;
+    float *edges = nullptr;
     std::uint32_t *order = nullptr;
     int rc = GWNB_OK;
     if (c->edge_count > 0) {
-        GWNB_TRY(alloc(&edges, 2 * c->edge_count, s));
-        note_launch(), k_edge_records<<<static_cast<unsigned>((c->edge_count + 255) / 256), 256, 0, s>>>(
+        std::uint64_t const pairs = (c->edge_count + 1) / 2;
+        GWNB_TRY(alloc(&edges, pairs * k_row_pair, s));
+        note_launch(), k_edge_records<<<static_cast<unsigned>((2 * pairs + 255) / 256), 256, 0, s>>>(
             *g, c->start_vertex, c->end_vertex, c->multiplicity, c->edge_count, edges);
     }
     if (o.sort_queries != 0 && n > 1 && a != nullptr) {
@@ -870,9 +1070,8 @@ static int antipodal_common(const gwnb_geometry_f32 *g, const gwnb_bvh4_f32 *b_i
             unsigned const grid = static_cast<unsigned>((n + block - 1) / block);
             note_launch(), k_antipodal_gradient<<<grid, block, 0, s>>>(p);
         } else {
-            std::uint64_t const per_block = static_cast<std::uint64_t>(block) * k_ap_q;
-            unsigned const grid = static_cast<unsigned>((n + per_block - 1) / per_block);
-            std::size_t const smem = 2 * k_ap_tile * sizeof(float4) +
+            unsigned const grid = static_cast<unsigned>((n + block - 1) / block);
+            std::size_t const smem = k_ap_tile / 2 * k_row_pair * sizeof(float) +
                                      static_cast<std::size_t>(p.stack_cap) * block * sizeof(std::uint32_t);
             cudaError_t e = cudaSuccess;
             if (smem > 48 * 1024)

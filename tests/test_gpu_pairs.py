@@ -1,4 +1,5 @@
-"""The exact batch takes its triangles two at a time: sizes around the edges of pairs, tiles and blocks, and queries that leave the
+"""The brute-force kernels take their records two at a time (triangles in the exact batch, boundary rows
+in the antipodal batch): sizes around the edges of pairs, tiles and blocks, and queries that leave the
 packed path (on vertices, in a triangle's plane, on an edge, on an edge's line, far away)."""
 from __future__ import annotations
 
@@ -6,7 +7,8 @@ import numpy as np
 import pytest
 
 import oracle
-from smallgwn_b200 import meshes
+from smallgwn_b200 import api, meshes
+from test_gpu_antipodal import chain_of, gpu_antipodal, gpu_gradient
 from test_gpu_build import build, upload
 from test_gpu_query import run_exact
 
@@ -63,3 +65,48 @@ def test_exact_batch_scales(cuda, scale):
     scaled = dict(mesh, **{k: (mesh[k] * np.float32(scale)).astype(np.float32) for k in "xyz"})
     got = run_exact(cuda, build(upload(scaled)), (q * np.float32(scale)).astype(np.float32))
     assert (np.abs(got - want) <= EXACT_TOL)[far].all()
+
+
+@pytest.mark.parametrize("triangles", [1, 2, 255, 400, 999])
+@pytest.mark.parametrize("n", [1, 257, 1000])
+def test_antipodal_batch_sizes(cuda, triangles, n):
+    mesh = part(triangles)
+    geo = upload(mesh)
+    bvh = build(geo)
+    ch = chain_of(geo)
+    h = api.bvh_host_arrays(bvh)
+    q = probes(mesh, n, seed=3 * triangles + n)
+    ref = oracle.antipodal(mesh, h["nodes"], h["triangles"], h["root_reference"], ch.rows(), *q)
+    got = gpu_antipodal(cuda, geo, bvh, ch, q)
+    np.testing.assert_array_equal(np.isnan(got), np.isnan(ref))
+    ok = ~np.isnan(ref)
+    assert np.abs(got[ok] - ref[ok]).max(initial=0.0) <= 2e-5  # as test_gpu_antipodal.test_equals_oracle
+    gr = gpu_gradient(cuda, geo, ch, q)
+    gref = oracle.antipodal_gradient(mesh, ch.rows(), *q)
+    np.testing.assert_array_equal(np.isnan(gr), np.isnan(gref))
+    # where the query is clear of the boundary (the gradient grows like the inverse of the distance, and
+    # float rounding of the query's offset with it): within 1e-5 of the largest
+    clear = ~np.isnan(gref).any(1) & (oracle.mesh_distance(mesh, *q) > 1e-2)
+    if clear.any():
+        assert np.abs(gr - gref)[clear].max() <= 1e-5 * max(1.0, float(np.abs(gref[clear]).max()))
+
+
+def test_rows_with_multiplicity(cuda):
+    """Three copies of one triangle: every boundary row has multiplicity 3."""
+    mesh = dict(part(1))
+    for k in ("i0", "i1", "i2"):
+        mesh[k] = np.repeat(mesh[k], 3)
+    single = part(1)
+    q = probes(single, 300, seed=4)
+    values, grads = [], []
+    for m in (single, mesh):
+        geo = upload(m)
+        ch = chain_of(geo)
+        values.append(gpu_antipodal(cuda, geo, build(geo), ch, q))
+        grads.append(gpu_gradient(cuda, geo, ch, q))
+    assert int(ch.rows()[2].max()) == 3
+    ok = np.isfinite(values[0])
+    np.testing.assert_allclose(values[1][ok], 3 * values[0][ok], rtol=1e-6, atol=1e-6)
+    # a row's gradient is at most 2 / (4 pi distance) of its edge: 16 here, rounded a few times (2^-24 each)
+    ok = np.isfinite(grads[0]).all(1) & (oracle.mesh_distance(single, *q) > 1e-2)
+    np.testing.assert_allclose(grads[1][ok], 3 * grads[0][ok], rtol=0, atol=3 * 16 * 8 * 2.0 ** -24)
