@@ -114,6 +114,7 @@ __global__ void __launch_bounds__(256, 4) k_adjoint_traverse(adjoint_params p) {
     float const qy = valid ? p.qy[qi] : 0.0f;
     float const qz = valid ? p.qz[qi] : 0.0f;
     float const gam = valid ? p.grad_out[qi] * (1.0f / (4.0f * k_pi_f)) : 0.0f;
+    x2::f2 const qx2 = x2::both(qx), qy2 = x2::both(qy), qz2 = x2::both(qz);
     bool const want_slots = p.slot_grad != nullptr;
     float dqx = 0.0f, dqy = 0.0f, dqz = 0.0f;
 
@@ -168,87 +169,93 @@ __global__ void __launch_bounds__(256, 4) k_adjoint_traverse(adjoint_params p) {
             std::uint32_t next = k_invalid_u32;
             unsigned next_mask = 0u;
 #pragma unroll 1
-            for (int s = 0; s < 4; ++s) {
-                float4 const a = __ldg(nd + s * Q);
-                if (a.w < 0.0f)
-                    continue;
-                float4 const b = __ldg(nd + s * Q + 1);
-                bool desc = false, acc = false;
-                float sv[SF];
+            for (int h = 0; h < 2; ++h) {
+                float4 const *w = nd + h * 2 * Q;
+                pair_head const hd = load_head(w, qx2, qy2, qz2, p.beta2);
+                bool const valid[2] = {hd.valid0, hd.valid1};
+                bool acc[2] = {active && hd.far0, active && hd.far1};
+                float sv[2][SF];
+                if (__any_sync(0xffffffffu, acc[0] || acc[1])) {
+                    x2::f2 g[3];
+                    float wv[2];
+                    x2::unpack(far_pair<Order, true>(hd, w, g[0], g[1], g[2]), wv[0], wv[1]);
+                    x2::f2 const k1 = x2::both(gam), m1 = x2::rsqrt(hd.q2), m2 = x2::mul(m1, m1);
+                    x2::f2 const n[3] = {x2::mul(hd.rx, m1), x2::mul(hd.ry, m1), x2::mul(hd.rz, m1)};
+                    x2::f2 v[SF];
+                    // dF/dN = -r^ / |r|^2; dF/dP = -dF/dq
+                    x2::f2 const kn = x2::mul(x2::both(-gam), m2);
 #pragma unroll
-                for (int j = 0; j < SF; ++j)
-                    sv[j] = 0.0f;
-                if (active) {
-                    float const rx = qx - a.x, ry = qy - a.y, rz = qz - a.z;
-                    float const q2 = accept_dist2(rx, ry, rz);
-                    desc = !far_accepted(q2, a.w, p.beta2);
-                    if (!desc) {
-                        float g0 = 0.0f, g1 = 0.0f, g2 = 0.0f;
-                        float const w = far_field<Order, true>(rx, ry, rz, q2, b, nd + s * Q + 2, g0, g1, g2);
-                        if (isfinite(w)) {
-                            acc = true;
-                            dqx += gam * g0;
-                            dqy += gam * g1;
-                            dqz += gam * g2;
-                            float const m1 = rsqrtf(q2);
-                            float const m2 = m1 * m1;
-                            float const nx = rx * m1, ny = ry * m1, nz = rz * m1;
-                            // dF/dN = -r^ / |r|^2; dF/dP = -dF/dq
-                            sv[0] = -gam * m2 * nx;
-                            sv[1] = -gam * m2 * ny;
-                            sv[2] = -gam * m2 * nz;
-                            sv[3] = -gam * g0;
-                            sv[4] = -gam * g1;
-                            sv[5] = -gam * g2;
-                            if constexpr (Order >= 1) {
-                                // dF/dM_ij = (delta_ij - 3 r^_i r^_j) / |r|^3
-                                float const k = gam * m2 * m1;
-                                sv[6] = k * (1.0f - 3.0f * nx * nx);
-                                sv[7] = k * (1.0f - 3.0f * ny * ny);
-                                sv[8] = k * (1.0f - 3.0f * nz * nz);
-                                sv[9] = -3.0f * k * nx * ny;
-                                sv[10] = -3.0f * k * ny * nz;
-                                sv[11] = -3.0f * k * nz * nx;
+                    for (int j = 0; j < 3; ++j) {
+                        v[j] = x2::mul(kn, n[j]);
+                        v[3 + j] = x2::mul(k1, g[j]);
+                    }
+                    if constexpr (Order >= 1) {
+                        // dF/dM_ij = (delta_ij - 3 r^_i r^_j) / |r|^3
+                        x2::f2 const k = x2::mul(k1, x2::mul(m2, m1));
+                        x2::f2 const k3 = x2::mul(k, x2::both(-3.0f));
+#pragma unroll
+                        for (int j = 0; j < 3; ++j) {
+                            x2::f2 const kj = x2::mul(k3, n[j]);
+                            v[6 + j] = x2::fma(kj, n[j], k);
+                            v[9 + j] = x2::mul(kj, n[j == 2 ? 0 : j + 1]);
+                        }
+                    }
+#pragma unroll
+                    for (int j = 0; j < SF; ++j)
+                        x2::unpack(v[j], sv[0][j], sv[1][j]);
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) {
+                        acc[c] = acc[c] && isfinite(wv[c]);
+                        dqx += acc[c] ? sv[c][3] : 0.0f;
+                        dqy += acc[c] ? sv[c][4] : 0.0f;
+                        dqz += acc[c] ? sv[c][5] : 0.0f;
+                        if (want_slots) {
+                            unsigned const amask = __ballot_sync(0xffffffffu, acc[c]);
+                            if (amask != 0u) {
+#pragma unroll
+                                for (int j = 0; j < SF; ++j)
+                                    sv[c][j] = acc[c] ? (j >= 3 && j < 6 ? -sv[c][j] : sv[c][j]) : 0.0f;
+                                warp_scatter_add<SF>(p.slot_grad + (static_cast<std::uint64_t>(node) * 4 + 2 * h + c) * SF,
+                                                     sv[c], amask, lane);
                             }
-                        } else {
-                            desc = true;
                         }
                     }
                 }
-                if (want_slots) {
-                    unsigned const amask = __ballot_sync(0xffffffffu, acc);
-                    if (amask != 0u)
-                        warp_scatter_add<SF>(p.slot_grad + (static_cast<std::uint64_t>(node) * 4 + s) * SF, sv,
-                                             amask, lane);
-                }
-                unsigned const dmask = __ballot_sync(0xffffffffu, desc);
-                if (dmask == 0u)
-                    continue;
-                std::uint32_t const ref = __float_as_uint(b.w);
-                if ((ref & k_qref_leaf) == 0u) {
-                    if (next != k_invalid_u32) {
-                        if (sp >= Cap) {
-                            overflow = true;
-                            break;
-                        }
-                        if (static_cast<unsigned>(sp & 31) == lane) {
-                            if (sp < 32) {
-                                st_node0 = next;
-                                st_mask0 = next_mask;
-                            } else {
-                                st_node1 = next;
-                                st_mask1 = next_mask;
+                std::uint32_t ref[2];
+                pair_refs(w, ref[0], ref[1]);
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    bool const desc = active && valid[c] && !acc[c];
+                    unsigned const dmask = __ballot_sync(0xffffffffu, desc);
+                    if (dmask == 0u)
+                        continue;
+                    if ((ref[c] & k_qref_leaf) == 0u) {
+                        if (next != k_invalid_u32) {
+                            if (sp >= Cap) {
+                                overflow = true;
+                                break;
                             }
+                            if (static_cast<unsigned>(sp & 31) == lane) {
+                                if (sp < 32) {
+                                    st_node0 = next;
+                                    st_mask0 = next_mask;
+                                } else {
+                                    st_node1 = next;
+                                    st_mask1 = next_mask;
+                                }
+                            }
+                            ++sp;
                         }
-                        ++sp;
+                        next = ref[c];
+                        next_mask = dmask;
+                    } else {
+                        std::uint32_t const cnt =
+                            (ref[c] & k_qref_multi) ? p.qcounts[static_cast<std::uint64_t>(node) * 4 + 2 * h + c] : 1u;
+                        leaf(ref[c] & k_qref_index_mask, cnt, desc, dmask);
                     }
-                    next = ref;
-                    next_mask = dmask;
-                } else {
-                    std::uint32_t const cnt =
-                        (ref & k_qref_multi) ? p.qcounts[static_cast<std::uint64_t>(node) * 4 + s] : 1u;
-                    leaf(ref & k_qref_index_mask, cnt, desc, dmask);
                 }
+                if (overflow)
+                    break;
             }
             if (overflow)
                 break;
@@ -367,9 +374,12 @@ __global__ void __launch_bounds__(256) k_adjoint_triangles(adjoint_tri_params p)
             atomicOr(p.status, k_err_topology);
             break;
         }
-        float4 const *sc = p.qnodes + (node * 4 + s) * Q;
-        float4 const a = __ldg(sc);     // P, r2
-        float4 const b = __ldg(sc + 1); // N, ref
+        // the slot's -P, r2, -N, ref from its pair
+        float4 const *w = p.qnodes + node * 4 * Q + (s >> 1) * 2 * Q;
+        float4 const w0 = __ldg(w), w1 = __ldg(w + 1), w2 = __ldg(w + 2), w3 = __ldg(w + 3);
+        bool const odd = (s & 1) != 0;
+        float3 const a = odd ? make_float3(-w0.y, -w0.w, -w1.y) : make_float3(-w0.x, -w0.z, -w1.x);
+        float4 const b = odd ? make_float4(-w2.y, -w2.w, -w3.y, w3.w) : make_float4(-w2.x, -w2.z, -w3.x, w3.z);
         float const *G = p.slot_grad + (node * 4 + s) * SF;
         float const dx = tt.cx - a.x, dy = tt.cy - a.y, dz = tt.cz - a.z;
         dnx += G[0];

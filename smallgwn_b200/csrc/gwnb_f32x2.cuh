@@ -42,6 +42,13 @@ __device__ __forceinline__ f2 fma(f2 a, f2 b, f2 c) {
     return r;
 }
 
+// Two packed values by one 128-bit read-only load.
+__device__ __forceinline__ void load(float4 const *p, f2 &a, f2 &b) {
+    ulonglong2 const v = __ldg(reinterpret_cast<ulonglong2 const *>(p));
+    a.v = v.x;
+    b.v = v.y;
+}
+
 // Reciprocal square root and reciprocal by the hardware's approximation alone (relative error below
 // 2^-22; denormals count as zero, so their results are infinite and what they reach becomes NaN).
 __device__ __forceinline__ float rsqrt_ftz(float x) {

@@ -12,6 +12,7 @@
 // (tr M - 3 r^T M r / |r|^2) / |r|^3 with M_ij = sum n_i (c - P)_j, order 2 the third-moment terms.
 #pragma once
 
+#include "gwnb_f32x2.cuh"
 #include "gwnb_internal.cuh"
 
 namespace gwnb {
@@ -19,19 +20,36 @@ namespace field {
 
 constexpr float k_pi_f = 3.14159265358979323846f;
 
-// |q - P|^2 for the acceptance test, with one fixed rounding pattern (rx * rx rounded, then two
-// fused multiply-adds) written out so that no compiler contraction choice can change it. Every
-// traversal (value, gradient, statistics, adjoint, batched) and the oracle's C restatement use
-// this pattern, so their accept / descend decisions are identical for identical inputs.
-__device__ __forceinline__ float accept_dist2(float rx, float ry, float rz) {
-    return __fmaf_rn(rz, rz, __fmaf_rn(ry, ry, __fmul_rn(rx, rx)));
-}
-
-// smallgwn's acceptance rule (detail/gwn_query_winding_impl.cuh:186-189): descend iff
-// !(|q - P|^2 > 0) or |q - P|^2 <= r^2 beta^2 (the product rounded on its own); a NaN bound
-// therefore accepts, as there.
-__device__ __forceinline__ bool far_accepted(float q2, float r2, float beta2) {
-    return q2 > 0.0f && !(q2 <= __fmul_rn(r2, beta2));
+// The head of a sidecar pair and the acceptance test of its two children. |q - P|^2 has one fixed
+// rounding pattern (rx * rx rounded, then two fused multiply-adds, r = q - P rounded per component), so
+// that every traversal (value, gradient, statistics, adjoint, batched) and the oracle's C restatement
+// take identical accept / descend decisions for identical inputs. The rule is smallgwn's
+// (detail/gwn_query_winding_impl.cuh:186-189): descend iff !(|q - P|^2 > 0) or |q - P|^2 <= r^2 beta^2
+// (the product rounded on its own); a NaN bound therefore accepts, as there.
+struct pair_head {
+    x2::f2 rx, ry, rz, q2; // r = q - P and |r|^2
+    bool valid0, valid1;   // slots that hold a child
+    bool far0, far1;       // ... and pass the acceptance test
+};
+__device__ __forceinline__ pair_head load_head(float4 const *w, x2::f2 qx, x2::f2 qy, x2::f2 qz, float beta2) {
+    using namespace x2;
+    pair_head h;
+    f2 px, py, pz, r2;
+    load(w, px, py);
+    load(w + 1, pz, r2);
+    h.rx = add(qx, px);
+    h.ry = add(qy, py);
+    h.rz = add(qz, pz);
+    h.q2 = dot(h.rx, h.ry, h.rz, h.rx, h.ry, h.rz);
+    float q0, q1, b0, b1, v0, v1;
+    unpack(h.q2, q0, q1);
+    unpack(mul(r2, both(beta2)), b0, b1);
+    unpack(r2, v0, v1);
+    h.valid0 = !(v0 < 0.0f);
+    h.valid1 = !(v1 < 0.0f);
+    h.far0 = h.valid0 && q0 > 0.0f && !(q0 <= b0);
+    h.far1 = h.valid1 && q1 > 0.0f && !(q1 <= b1);
+    return h;
 }
 
 // a = v0 - q, e1, e2 edges, n = e1 x e2.
@@ -250,79 +268,108 @@ __device__ __forceinline__ vertex_grad solid_angle_vertex_grad(float ax, float a
     return r;
 }
 
-// Far-field Taylor terms of one accepted child: smallgwn's expansion
-// (gwn_query_winding_impl.cuh:193-327) on the folded sidecar coefficients the moment refit writes.
-// r = q - P, q2 = |r|^2, n = r / |r|; b = (N, ref); cd.. = order-1 quadratic form M' (xx yy zz xy yz
-// zx) then order-2 cubic form K (xxx yyy zzz xxy xxz yyx yyz zzx zzy xyz):
+// Far-field Taylor terms of the two children of a sidecar pair: smallgwn's expansion
+// (gwn_query_winding_impl.cuh:193-327) on the folded coefficients the moment refit writes. r = q - P,
+// n = r / |r|; the quadratic form M' over xx yy zz xy yz zx, the cubic form K over xxx yyy zzz xxy xxz yyx
+// yyz zzx zzy xyz:
 //   w = -(n.N) / |r|^2 + n^T M' n / |r|^3 + K(n,n,n) / |r|^4.
 // With Grad, g is the derivative with respect to the query: the terms are P(r) / |r|^(2p+1) for
-// homogeneous P of degree p = 1, 2, 3, whose gradient is (grad P(n) - (2p+1) P(n) n) / |r|^(p+2).
+// homogeneous P of degree p = 1, 2, 3, whose gradient is (grad P(n) - (2p+1) P(n) n) / |r|^(p+2), and
+// P(n) = n . grad P(n) / p. One child's |r|^2 may be anything (its result is then not used); one that
+// underflows to the denormals gives a result that is not finite, and its child is entered.
 template <int Order, bool Grad>
-__device__ __forceinline__ float far_field(float rx, float ry, float rz, float q2, float4 const &b,
-                                           float4 const *__restrict__ cd, float &g0, float &g1, float &g2) {
-    float const m1 = rsqrtf(q2);
-    float const m2 = m1 * m1;
-    float const m3 = m2 * m1;
-    float const nx = rx * m1, ny = ry * m1, nz = rz * m1;
-    float const rdn = nx * b.x + ny * b.y + nz * b.z;
-    float w = -m2 * rdn;
-    if constexpr (Grad) {
-        g0 = m3 * (3.0f * nx * rdn - b.x);
-        g1 = m3 * (3.0f * ny * rdn - b.y);
-        g2 = m3 * (3.0f * nz * rdn - b.z);
-    }
-    if constexpr (Order >= 1 && !Grad) {
-        // value only: the forms factored by components (Q1 in 7 and Q2 in 13 operations on the
-        // shared squares), grouped explicitly since the compiler keeps the written FP order
-        float4 const c = __ldg(cd);
-        float4 const d = __ldg(cd + 1);
-        float const xx = nx * nx, yy = ny * ny, zz = nz * nz, yz = ny * nz;
-        float const Q1 = c.x * xx + c.y * yy + c.z * zz + d.x * yz + nx * (c.w * ny + d.y * nz);
-        float t = Q1;
-        if constexpr (Order >= 2) {
-            float4 const e = __ldg(cd + 2);
-            float4 const f = __ldg(cd + 3);
-            float const Q2 = nx * (d.z * xx + e.w * yy + f.y * zz + f.w * yz) + ny * (d.w * yy + e.y * xx + f.z * zz) +
-                             nz * (e.x * zz + e.z * xx + f.x * yy);
-            t += m1 * Q2;
+__device__ __forceinline__ x2::f2 far_pair(pair_head const &h, float4 const *w, x2::f2 &g0, x2::f2 &g1, x2::f2 &g2) {
+    using namespace x2;
+    f2 const m1 = rsqrt(h.q2);
+    f2 const m2 = mul(m1, m1);
+    f2 const x = mul(h.rx, m1), y = mul(h.ry, m1), z = mul(h.rz, m1);
+    f2 Nx, Ny, Nz, ref; // -N
+    load(w + 2, Nx, Ny);
+    load(w + 3, Nz, ref);
+    f2 const t0 = dot(x, y, z, Nx, Ny, Nz); // -(n.N)
+    if constexpr (!Grad) {
+        if constexpr (Order == 0) {
+            return mul(m2, t0);
+        } else {
+            // the forms factored by components: M' in 7 and K in 13 operations on the shared squares
+            f2 cxx, cyy, czz, cxy, cyz, czx;
+            load(w + 4, cxx, cyy);
+            load(w + 5, czz, cxy);
+            load(w + 6, cyz, czx);
+            f2 const xx = mul(x, x), yy = mul(y, y), zz = mul(z, z), yz = mul(y, z);
+            f2 t = fma(cyz, yz, fma(czz, zz, fma(cyy, yy, mul(cxx, xx))));
+            t = fma(x, fma(czx, z, mul(cxy, y)), t);
+            if constexpr (Order >= 2) {
+                f2 kxxx, kyyy, kzzz, kxxy, kxxz, kyyx, kyyz, kzzx, kzzy, kxyz;
+                load(w + 7, kxxx, kyyy);
+                load(w + 8, kzzz, kxxy);
+                load(w + 9, kxxz, kyyx);
+                load(w + 10, kyyz, kzzx);
+                load(w + 11, kzzy, kxyz);
+                f2 q = mul(x, fma(kxyz, yz, fma(kzzx, zz, fma(kyyx, yy, mul(kxxx, xx)))));
+                q = fma(y, fma(kzzy, zz, fma(kxxy, xx, mul(kyyy, yy))), q);
+                q = fma(z, fma(kyyz, yy, fma(kxxz, xx, mul(kzzz, zz))), q);
+                t = fma(m1, q, t);
+            }
+            return mul(m2, fma(m1, t, t0));
         }
-        w += m3 * t;
-        return w;
-    }
-    if constexpr (Order >= 1) {
-        float4 const c = __ldg(cd);
-        float4 const d = __ldg(cd + 1);
-        float const xx = nx * nx, yy = ny * ny, zz = nz * nz, xy = nx * ny, yz = ny * nz, zx = nz * nx;
-        float const Q1 = c.x * xx + c.y * yy + c.z * zz + c.w * xy + d.x * yz + d.y * zx;
-        w += m3 * Q1;
-        if constexpr (Grad) {
-            float const m4 = m2 * m2;
-            float const k = 5.0f * Q1;
-            g0 += m4 * (2.0f * c.x * nx + c.w * ny + d.y * nz - k * nx);
-            g1 += m4 * (c.w * nx + 2.0f * c.y * ny + d.x * nz - k * ny);
-            g2 += m4 * (d.y * nx + d.x * ny + 2.0f * c.z * nz - k * nz);
-        }
-        if constexpr (Order >= 2) {
-            float4 const e = __ldg(cd + 2);
-            float4 const f = __ldg(cd + 3);
-            // K over xxx yyy zzz xxy | xxz yyx yyz zzx | zzy xyz
-            float const Q2 = d.z * xx * nx + d.w * yy * ny + e.x * zz * nz + e.y * xx * ny + e.z * xx * nz +
-                             e.w * yy * nx + f.x * yy * nz + f.y * zz * nx + f.z * zz * ny + f.w * xy * nz;
-            float const m4 = m2 * m2;
-            w += m4 * Q2;
-            if constexpr (Grad) {
-                float const m5 = m4 * m1;
-                float const k = 7.0f * Q2;
-                float const Gx = 3.0f * d.z * xx + 2.0f * e.y * xy + 2.0f * e.z * zx + e.w * yy + f.y * zz + f.w * yz;
-                float const Gy = 3.0f * d.w * yy + e.y * xx + 2.0f * e.w * xy + 2.0f * f.x * yz + f.z * zz + f.w * zx;
-                float const Gz = 3.0f * e.x * zz + e.z * xx + f.x * yy + 2.0f * f.y * zx + 2.0f * f.z * yz + f.w * xy;
-                g0 += m5 * (Gx - k * nx);
-                g1 += m5 * (Gy - k * ny);
-                g2 += m5 * (Gz - k * nz);
+    } else {
+        f2 const m3 = mul(m2, m1);
+        f2 gx = Nx, gy = Ny, gz = Nz;       // grad P(n) / |r|^(p-1), summed
+        f2 s = mul(t0, both(-3.0f));        // sum of -(2p+1) P(n) / |r|^(p-1)
+        f2 value = t0;                      // sum of P(n) / |r|^(p-1)
+        if constexpr (Order >= 1) {
+            f2 cxx, cyy, czz, cxy, cyz, czx;
+            load(w + 4, cxx, cyy);
+            load(w + 5, czz, cxy);
+            load(w + 6, cyz, czx);
+            f2 const two = both(2.0f);
+            f2 const dx = fma(mul(cxx, two), x, fma(cxy, y, mul(czx, z)));
+            f2 const dy = fma(mul(cyy, two), y, fma(cxy, x, mul(cyz, z)));
+            f2 const dz = fma(mul(czz, two), z, fma(cyz, y, mul(czx, x)));
+            f2 const q1 = mul(m1, dot(x, y, z, dx, dy, dz)); // 2 P / |r|
+            gx = fma(m1, dx, gx);
+            gy = fma(m1, dy, gy);
+            gz = fma(m1, dz, gz);
+            s = fma(q1, both(-2.5f), s);
+            value = fma(q1, both(0.5f), value);
+            if constexpr (Order >= 2) {
+                f2 kxxx, kyyy, kzzz, kxxy, kxxz, kyyx, kyyz, kzzx, kzzy, kxyz;
+                load(w + 7, kxxx, kyyy);
+                load(w + 8, kzzz, kxxy);
+                load(w + 9, kxxz, kyyx);
+                load(w + 10, kyyz, kzzx);
+                load(w + 11, kzzy, kxyz);
+                f2 const xx = mul(x, x), yy = mul(y, y), zz = mul(z, z);
+                f2 const x2_ = mul(x, two), y2_ = mul(y, two), xy = mul(x2_, y), yz = mul(y2_, z), zx = mul(x2_, z);
+                f2 const three = both(3.0f), half = both(0.5f);
+                f2 const ex = fma(mul(kxxx, three), xx,
+                                  fma(kxxy, xy, fma(kxxz, zx, fma(kyyx, yy, fma(kzzx, zz, mul(mul(kxyz, half), yz))))));
+                f2 const ey = fma(mul(kyyy, three), yy,
+                                  fma(kyyx, xy, fma(kyyz, yz, fma(kxxy, xx, fma(kzzy, zz, mul(mul(kxyz, half), zx))))));
+                f2 const ez = fma(mul(kzzz, three), zz,
+                                  fma(kzzx, zx, fma(kzzy, yz, fma(kxxz, xx, fma(kyyz, yy, mul(mul(kxyz, half), xy))))));
+                f2 const q2 = mul(m2, dot(x, y, z, ex, ey, ez)); // 3 P / |r|^2
+                gx = fma(m2, ex, gx);
+                gy = fma(m2, ey, gy);
+                gz = fma(m2, ez, gz);
+                s = fma(q2, both(-7.0f / 3.0f), s);
+                value = fma(q2, both(1.0f / 3.0f), value);
             }
         }
+        g0 = mul(m3, fma(s, x, gx));
+        g1 = mul(m3, fma(s, y, gy));
+        g2 = mul(m3, fma(s, z, gz));
+        return mul(m2, value);
     }
-    return w;
+}
+
+// Child references of a pair.
+__device__ __forceinline__ void pair_refs(float4 const *w, std::uint32_t &r0, std::uint32_t &r1) {
+    x2::f2 nz, ref;
+    x2::load(w + 3, nz, ref);
+    r0 = static_cast<std::uint32_t>(ref.v);
+    r1 = static_cast<std::uint32_t>(ref.v >> 32);
 }
 
 } // namespace field

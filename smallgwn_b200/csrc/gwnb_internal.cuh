@@ -108,10 +108,12 @@ __host__ __device__ inline std::uint64_t make_ref(std::uint64_t offset, std::uin
     return k_valid_bit | offset | (count << k_count_shift);
 }
 
-// Query sidecar (one record per wide node, written by the moment refit). Per child slot the
-// record holds float4 blocks: a = (P.xyz, r2) with r2 < 0 marking an invalid slot,
-// b = (N.xyz, ref bits), then the folded far-field coefficients (order 1: the 6 entries of
-// M' = trace(M) I - 3M; order 2: those 6 and the 10 of the cubic form K). ref bits: internal child -> node index;
+// Query sidecar (one record per wide node, written by the moment refit): the child slots in two pairs
+// (0, 1) and (2, 3), a pair's components interleaved -- (component 0 of the even slot, of the odd one),
+// (component 1 of ...) -- so that one 128-bit load brings two components of both children as operands of
+// packed FP32 instructions. Components: -P (xyz), r2 (negative: invalid slot), -N (xyz), ref bits, then
+// the folded far-field coefficients (order 1: the 6 entries of M' = trace(M) I - 3M; order 2: those 6
+// and the 10 of the cubic form K), padded to a multiple of four. ref bits: internal child -> node index;
 // leaf -> 0x80000000 | first sorted triangle; bit 30 set when the leaf holds more than one
 // triangle (its count is then read from the per-node count table).
 constexpr std::uint32_t k_qref_leaf = 0x80000000u;
@@ -122,6 +124,11 @@ template <int Order> struct qnode_traits;
 template <> struct qnode_traits<0> { static constexpr int k_f4_per_child = 2; };
 template <> struct qnode_traits<1> { static constexpr int k_f4_per_child = 4; };
 template <> struct qnode_traits<2> { static constexpr int k_f4_per_child = 6; };
+// Components of a child slot, and the place of component c of slot s in a node's record (in floats).
+template <int Order> constexpr int k_qnode_components = 4 * qnode_traits<Order>::k_f4_per_child;
+template <int Order> __host__ __device__ constexpr int qnode_at(int s, int c) {
+    return (s >> 1) * 2 * k_qnode_components<Order> + 2 * c + (s & 1);
+}
 inline int qnode_f4_per_child(int order) { return order == 0 ? 2 : (order == 1 ? 4 : 6); }
 
 // Field counts of smallgwn's moment node (floats per child slot).

@@ -329,6 +329,37 @@ struct taylor_params {
     unsigned int *status;
 };
 
+// Adds the far fields of a pair's children that f0 and f1 name, even slot first; clears the flag of a
+// child whose expansion is not finite (it is entered instead).
+template <int Order, int Mode, bool Grad, bool Stats>
+__device__ __forceinline__ void add_far_pair(pair_head const &hd, float4 const *w, bool &f0, bool &f1,
+                                             accum<Mode == GWNB_NEAR_COMPENSATED> &omega, float &gx, float &gy,
+                                             float &gz, std::uint32_t &st_far) {
+    x2::f2 g0, g1, g2;
+    float w0, w1;
+    x2::unpack(far_pair<Order, Grad>(hd, w, g0, g1, g2), w0, w1);
+    f0 = f0 && isfinite(w0);
+    f1 = f1 && isfinite(w1);
+    if (f0)
+        omega.add(w0);
+    if (f1)
+        omega.add(w1);
+    if constexpr (Grad) {
+        float a0, a1, b0, b1, c0, c1;
+        x2::unpack(g0, a0, a1);
+        x2::unpack(g1, b0, b1);
+        x2::unpack(g2, c0, c1);
+        gx += f0 ? a0 : 0.0f;
+        gy += f0 ? b0 : 0.0f;
+        gz += f0 ? c0 : 0.0f;
+        gx += f1 ? a1 : 0.0f;
+        gy += f1 ? b1 : 0.0f;
+        gz += f1 ? c1 : 0.0f;
+    }
+    if constexpr (Stats)
+        st_far += (f0 ? 1u : 0u) + (f1 ? 1u : 0u);
+}
+
 // One query of the per-thread traversal: sorted position idx of the batch described by p, with
 // s_stack pointing at this thread's column of a [Cap][blockDim.x] shared-memory stack.
 template <int Order, int Cap, int Mode, bool Grad, bool Stats>
@@ -340,6 +371,7 @@ __device__ __forceinline__ void taylor_thread_item(taylor_params const &p, std::
     std::uint32_t const qi = p.order != nullptr ? p.order[idx] : static_cast<std::uint32_t>(idx);
     std::uint64_t const li = p.gathered ? idx : qi;
     float const qx = p.qx[li], qy = p.qy[li], qz = p.qz[li];
+    x2::f2 const qx2 = x2::both(qx), qy2 = x2::both(qy), qz2 = x2::both(qz);
     accum<Mode == GWNB_NEAR_COMPENSATED> omega;
     float gx = 0.0f, gy = 0.0f, gz = 0.0f;
     std::uint32_t st_nodes = 0, st_far = 0, st_near = 0;
@@ -386,44 +418,39 @@ __device__ __forceinline__ void taylor_thread_item(taylor_params const &p, std::
             float4 const *nd = p.qnodes + static_cast<std::uint64_t>(node) * (4 * Q);
             std::uint32_t next = k_invalid_u32;
 #pragma unroll
-            for (int s = 0; s < 4; ++s) {
-                float4 const a = __ldg(nd + s * Q);
-                if (a.w < 0.0f)
+            for (int h = 0; h < 2; ++h) {
+                float4 const *w = nd + h * 2 * Q;
+                pair_head const hd = load_head(w, qx2, qy2, qz2, p.beta2);
+                bool f0 = hd.far0, f1 = hd.far1;
+                if (f0 || f1)
+                    add_far_pair<Order, Mode, Grad, Stats>(hd, w, f0, f1, omega, gx, gy, gz, st_far);
+                if ((!hd.valid0 || f0) && (!hd.valid1 || f1))
                     continue;
-                float4 const b = __ldg(nd + s * Q + 1);
-                float const rx = qx - a.x, ry = qy - a.y, rz = qz - a.z;
-                float const q2 = accept_dist2(rx, ry, rz);
-                bool descend = !far_accepted(q2, a.w, p.beta2);
-                if (!descend) {
-                    float g0 = 0.0f, g1 = 0.0f, g2 = 0.0f;
-                    float const w = far_field<Order, Grad>(rx, ry, rz, q2, b, nd + s * Q + 2, g0, g1, g2);
-                    if (isfinite(w)) {
-                        omega.add(w);
-                        if constexpr (Grad) {
-                            gx += g0;
-                            gy += g1;
-                            gz += g2;
-                        }
-                        if constexpr (Stats)
-                            ++st_far;
+                std::uint32_t ref[2];
+                pair_refs(w, ref[0], ref[1]);
+                bool const desc[2] = {hd.valid0 && !f0, hd.valid1 && !f1};
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    if (!desc[c])
                         continue;
-                    }
-                }
-                std::uint32_t const ref = __float_as_uint(b.w);
-                if ((ref & k_qref_leaf) == 0u) {
-                    if (next != k_invalid_u32) {
-                        if (sp >= cap) {
-                            overflow = true;
-                            break;
+                    if ((ref[c] & k_qref_leaf) == 0u) {
+                        if (next != k_invalid_u32) {
+                            if (sp >= cap) {
+                                overflow = true;
+                                break;
+                            }
+                            stack[static_cast<unsigned>(sp) * stride] = next;
+                            ++sp;
                         }
-                        stack[static_cast<unsigned>(sp) * stride] = next;
-                        ++sp;
+                        next = ref[c];
+                    } else {
+                        std::uint32_t const cnt =
+                            (ref[c] & k_qref_multi) ? p.qcounts[static_cast<std::uint64_t>(node) * 4 + 2 * h + c] : 1u;
+                        leaf(ref[c] & k_qref_index_mask, cnt);
                     }
-                    next = ref;
-                } else {
-                    std::uint32_t const cnt = (ref & k_qref_multi) ? p.qcounts[static_cast<std::uint64_t>(node) * 4 + s] : 1u;
-                    leaf(ref & k_qref_index_mask, cnt);
                 }
+                if (overflow)
+                    break;
             }
             if (overflow)
                 break;
@@ -477,14 +504,18 @@ __global__ void __launch_bounds__(256) k_taylor(taylor_params p) {
 // loaded with warp-uniform addresses and the stack lives in the lanes' registers (lane k holds
 // entries k and k + 32), so control flow stays uniform. For every lane the nodes it needs are
 // visited in the same order as in an independent depth-first traversal (children in decreasing
-// slot order, contributions added in slot order), so the per-lane sums equal those of k_taylor.
-// Occupancy: the plain form fits 48 registers (5 resident blocks of 256); the compensated near
-// field would take ~70, so it is bounded to 4 blocks (64 registers) and the rarely taken FP64 branch
-// absorbs any spilling; the gradient and statistics forms also take 4, and the compensated gradient
-// 3 (85 registers).
-template <int Mode, bool Grad, bool Stats> struct taylor_warp_occupancy {
+// slot order, contributions of a pair added far field first), so the per-lane sums equal those of
+// k_taylor. Bound by instruction issue: the four children are taken in two pairs, their tests and far
+// fields in packed instructions for both (70 % of the children a lane meets are accepted, so little of
+// the second half is wasted), and a pair's votes, loads and branches are shared. 10M surface-heavy
+// queries on a 1M-triangle sphere, order 2, compensated: 35.8 ms child by child, 31.8 ms in pairs; 1M
+// mixed queries, order 1, plain: 2.03 and 1.64 ms.
+// Occupancy: the plain form of orders 0 and 1 fits 48 registers (5 resident blocks of 256); a pair of
+// children's 24 order-2 components, the compensated near field and the gradient and statistics forms take
+// 64 (4 blocks), the gradient of order 2 or with the compensated near field 80 (3 blocks).
+template <int Order, int Mode, bool Grad, bool Stats> struct taylor_warp_occupancy {
     static constexpr bool comp = Mode == GWNB_NEAR_COMPENSATED;
-    static constexpr int value = (comp && Grad) ? 3 : ((comp || Grad || Stats) ? 4 : 5);
+    static constexpr int value = (Grad && (comp || Order == 2)) ? 3 : ((comp || Grad || Stats || Order == 2) ? 4 : 5);
 };
 
 // Block shape of the single-BVH warp kernel. The block size changes no result (every warp walks
@@ -492,10 +523,10 @@ template <int Mode, bool Grad, bool Stats> struct taylor_warp_occupancy {
 // 8 blocks of 128 (the same 32 warps and 64 registers as 4 of 256, but a block's warp slots come
 // free when its 4 warps are done rather than 8; 1 % less kernel time on the 10M-query workload),
 // the other forms blocks of 256.
-template <int Mode, bool Grad, bool Stats> struct taylor_warp_shape {
+template <int Order, int Mode, bool Grad, bool Stats> struct taylor_warp_shape {
     static constexpr bool small = Mode == GWNB_NEAR_COMPENSATED && !Grad && !Stats;
     static constexpr int block = small ? 128 : 256;
-    static constexpr int blocks = small ? 8 : taylor_warp_occupancy<Mode, Grad, Stats>::value;
+    static constexpr int blocks = small ? 8 : taylor_warp_occupancy<Order, Mode, Grad, Stats>::value;
 };
 
 // One warp of the warp-cooperative traversal: lane k takes sorted position idx (idx - lane is the
@@ -517,6 +548,7 @@ __device__ __forceinline__ void taylor_warp_item(taylor_params const &p, std::ui
     float const qx = valid ? p.qx[li] : 0.0f;
     float const qy = valid ? p.qy[li] : 0.0f;
     float const qz = valid ? p.qz[li] : 0.0f;
+    x2::f2 const qx2 = x2::both(qx), qy2 = x2::both(qy), qz2 = x2::both(qz);
     accum<Mode == GWNB_NEAR_COMPENSATED> omega;
     float gx = 0.0f, gy = 0.0f, gz = 0.0f;
     std::uint32_t st_nodes = 0, st_far = 0, st_near = 0;
@@ -570,66 +602,52 @@ __device__ __forceinline__ void taylor_warp_item(taylor_params const &p, std::ui
             std::uint32_t next = k_invalid_u32;
             unsigned next_mask = 0u;
 #pragma unroll
-            for (int s = 0; s < 4; ++s) {
-                float4 const a = __ldg(nd + s * Q);
-                if (a.w < 0.0f)
+            for (int h = 0; h < 2; ++h) {
+                float4 const *w = nd + h * 2 * Q;
+                pair_head const hd = load_head(w, qx2, qy2, qz2, p.beta2);
+                bool f0 = active && hd.far0, f1 = active && hd.far1;
+                if (__any_sync(0xffffffffu, f0 || f1))
+                    add_far_pair<Order, Mode, Grad, Stats>(hd, w, f0, f1, omega, gx, gy, gz, st_far);
+                bool const desc[2] = {active && hd.valid0 && !f0, active && hd.valid1 && !f1};
+                unsigned const dmask[2] = {__ballot_sync(0xffffffffu, desc[0]), __ballot_sync(0xffffffffu, desc[1])};
+                if ((dmask[0] | dmask[1]) == 0u)
                     continue;
-                float4 const b = __ldg(nd + s * Q + 1);
-                bool desc = false;
-                if (active) {
-                    float const rx = qx - a.x, ry = qy - a.y, rz = qz - a.z;
-                    float const q2 = accept_dist2(rx, ry, rz);
-                    desc = !far_accepted(q2, a.w, p.beta2);
-                    if (!desc) {
-                        float g0 = 0.0f, g1 = 0.0f, g2 = 0.0f;
-                        float const w = far_field<Order, Grad>(rx, ry, rz, q2, b, nd + s * Q + 2, g0, g1, g2);
-                        if (isfinite(w)) {
-                            omega.add(w);
-                            if constexpr (Grad) {
-                                gx += g0;
-                                gy += g1;
-                                gz += g2;
+                std::uint32_t ref[2];
+                pair_refs(w, ref[0], ref[1]);
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    if (dmask[c] == 0u)
+                        continue;
+                    if ((ref[c] & k_qref_leaf) == 0u) {
+                        if (next != k_invalid_u32) {
+                            if (sp >= Cap) {
+                                overflow = true;
+                                break;
                             }
-                            if constexpr (Stats)
-                                ++st_far;
-                        } else {
-                            desc = true;
-                        }
-                    }
-                }
-                unsigned const dmask = __ballot_sync(0xffffffffu, desc);
-                if (dmask == 0u)
-                    continue;
-                std::uint32_t const ref = __float_as_uint(b.w);
-                if ((ref & k_qref_leaf) == 0u) {
-                    if (next != k_invalid_u32) {
-                        if (sp >= Cap) {
-                            overflow = true;
-                            break;
-                        }
-                        if (static_cast<unsigned>(sp & 31) == lane) {
-                            if (sp < 32) {
-                                st_node0 = next;
-                                st_mask0 = next_mask;
-                            } else {
-                                st_node1 = next;
-                                st_mask1 = next_mask;
+                            if (static_cast<unsigned>(sp & 31) == lane) {
+                                if (sp < 32) {
+                                    st_node0 = next;
+                                    st_mask0 = next_mask;
+                                } else {
+                                    st_node1 = next;
+                                    st_mask1 = next_mask;
+                                }
                             }
+                            ++sp;
                         }
-                        ++sp;
-                    }
-                    next = ref;
-                    next_mask = dmask;
-                } else {
-                    if constexpr (Stats) // the warp runs the leaf loop for its descending lanes
-                        st_union_near +=
-                            (ref & k_qref_multi) ? p.qcounts[static_cast<std::uint64_t>(node) * 4 + s] : 1u;
-                    if (desc) {
+                        next = ref[c];
+                        next_mask = dmask[c];
+                    } else {
                         std::uint32_t const cnt =
-                            (ref & k_qref_multi) ? p.qcounts[static_cast<std::uint64_t>(node) * 4 + s] : 1u;
-                        leaf(ref & k_qref_index_mask, cnt);
+                            (ref[c] & k_qref_multi) ? p.qcounts[static_cast<std::uint64_t>(node) * 4 + 2 * h + c] : 1u;
+                        if constexpr (Stats) // the warp runs the leaf loop for its descending lanes
+                            st_union_near += cnt;
+                        if (desc[c])
+                            leaf(ref[c] & k_qref_index_mask, cnt);
                     }
                 }
+                if (overflow)
+                    break;
             }
             if (overflow)
                 break;
@@ -700,8 +718,8 @@ __device__ __forceinline__ void taylor_warp_item(taylor_params const &p, std::ui
 }
 
 template <int Order, int Cap, int Mode, bool Grad, bool Stats>
-__global__ void __launch_bounds__((taylor_warp_shape<Mode, Grad, Stats>::block),
-                                  (taylor_warp_shape<Mode, Grad, Stats>::blocks))
+__global__ void __launch_bounds__((taylor_warp_shape<Order, Mode, Grad, Stats>::block),
+                                  (taylor_warp_shape<Order, Mode, Grad, Stats>::blocks))
     k_taylor_warp(taylor_params p) {
     taylor_warp_item<Order, Cap, Mode, Grad, Stats>(p, static_cast<std::uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x);
 }
@@ -726,7 +744,7 @@ __device__ __forceinline__ std::uint32_t find_mesh_warp(std::uint64_t const *beg
 }
 
 template <int Order, int Cap, int Mode>
-__global__ void __launch_bounds__(256, (taylor_warp_occupancy<Mode, false, false>::value))
+__global__ void __launch_bounds__(256, (taylor_warp_occupancy<Order, Mode, false, false>::value))
     k_batch_taylor_warp(taylor_params const *__restrict__ meshes, std::uint64_t const *__restrict__ warp_begin,
                         std::uint32_t mesh_count, std::uint64_t warps) {
     std::uint64_t const warps_per_grid = static_cast<std::uint64_t>(gridDim.x) * (blockDim.x >> 5);
@@ -753,7 +771,7 @@ __global__ void __launch_bounds__(256)
 
 template <int Order, int Cap, int Mode, bool Grad, bool Stats>
 int launch_taylor_warp(taylor_params const &p, cudaStream_t s) {
-    constexpr int block = taylor_warp_shape<Mode, Grad, Stats>::block;
+    constexpr int block = taylor_warp_shape<Order, Mode, Grad, Stats>::block;
     unsigned const grid = static_cast<unsigned>((p.n + block - 1) / block);
     note_launch(), k_taylor_warp<Order, Cap, Mode, Grad, Stats><<<grid, block, 0, s>>>(p);
     GWNB_CUDA_TRY(cudaGetLastError());

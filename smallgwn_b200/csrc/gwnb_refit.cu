@@ -550,8 +550,10 @@ template <int Order> __device__ inline payload<Order> load_payload_cg(payload<Or
     return v;
 }
 
+// s_even is this thread's column of a [k_qnode_components][blockDim.x] shared-memory array: the even
+// slot's sidecar components wait there for the odd slot's, so that a pair is stored in 128-bit words.
 template <int Order>
-__device__ inline void finish_node(moment_params const &p, std::uint32_t n) {
+__device__ inline void finish_node(moment_params const &p, std::uint32_t n, float *s_even) {
     constexpr int F = Order == 0 ? 7 : (Order == 1 ? 13 : 23);
     constexpr int Q = qnode_traits<Order>::k_f4_per_child;
     payload<Order> *pend = static_cast<payload<Order> *>(p.pending);
@@ -609,14 +611,13 @@ __device__ inline void finish_node(moment_params const &p, std::uint32_t n) {
 #pragma unroll
             for (int f = 0; f < F; ++f)
                 ref[f * 4 + s] = c.f[f];
-            // sidecar: a = (P, r2), b = (N, ref), then coefficients 7.. in order
-            q[0] = c.f[1];
-            q[1] = c.f[2];
-            q[2] = c.f[3];
+            q[0] = -c.f[1];
+            q[1] = -c.f[2];
+            q[2] = -c.f[3];
             q[3] = c.f[0];
-            q[4] = c.f[4];
-            q[5] = c.f[5];
-            q[6] = c.f[6];
+            q[4] = -c.f[4];
+            q[5] = -c.f[5];
+            q[6] = -c.f[6];
             q[7] = __uint_as_float(qref);
             if constexpr (Order >= 1)
                 fold_far_field_coefficients<Order>(c, q + 8);
@@ -626,16 +627,24 @@ __device__ inline void finish_node(moment_params const &p, std::uint32_t n) {
                 total = m;
             init = true;
         }
+        if ((s & 1) == 0) {
 #pragma unroll
-        for (int k = 0; k < Q; ++k)
-            qn[s * Q + k] = make_float4(q[4 * k], q[4 * k + 1], q[4 * k + 2], q[4 * k + 3]);
+            for (int k = 0; k < Q * 4; ++k)
+                s_even[k * blockDim.x] = q[k];
+        } else {
+#pragma unroll
+            for (int k = 0; k < Q * 2; ++k)
+                qn[(s >> 1) * 2 * Q + k] = make_float4(s_even[2 * k * blockDim.x], q[2 * k],
+                                                       s_even[(2 * k + 1) * blockDim.x], q[2 * k + 1]);
+        }
     }
     store_payload_cg(pend + n, total);
 }
 
 // One work item of the moment refit: from leaf-bearing node t, finish every node this thread is
 // the last arrival at, climbing to the root.
-template <int Order> __device__ __forceinline__ void refit_moments_item(moment_params const &p, std::uint64_t t) {
+template <int Order>
+__device__ __forceinline__ void refit_moments_item(moment_params const &p, std::uint64_t t, float *s_even) {
     std::uint32_t cur = p.leaf_nodes[t];
     std::uint64_t guard = 0;
     for (;;) {
@@ -650,7 +659,7 @@ template <int Order> __device__ __forceinline__ void refit_moments_item(moment_p
         }
         p.arrivals[cur] = 0u;
         fence_acq_rel_gpu();
-        finish_node<Order>(p, cur);
+        finish_node<Order>(p, cur, s_even);
         std::uint32_t const ps = p.parent_slot[cur];
         if (ps == k_invalid_u32)
             return;
@@ -664,9 +673,10 @@ template <int Order> __device__ __forceinline__ void refit_moments_item(moment_p
 }
 
 template <int Order> __global__ void __launch_bounds__(k_block) k_refit_moments(moment_params p) {
+    __shared__ float s_even[k_qnode_components<Order> * k_block];
     std::uint64_t const t = static_cast<std::uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t < p.leaf_node_count)
-        refit_moments_item<Order>(p, t);
+        refit_moments_item<Order>(p, t, s_even + threadIdx.x);
 }
 
 // ---- batched refit (many BVHs, one launch) -------------------------------------------------------
@@ -716,11 +726,12 @@ template <int Order>
 __global__ void __launch_bounds__(k_batch_block_max)
     k_batch_refit_moments(moment_params const *__restrict__ meshes, std::uint64_t const *__restrict__ begin,
                           std::uint32_t mesh_count) {
+    __shared__ float s_even[k_qnode_components<Order> * k_batch_block_max];
     std::uint64_t const total = begin[mesh_count];
     for (std::uint64_t i = static_cast<std::uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
          i += static_cast<std::uint64_t>(gridDim.x) * blockDim.x) {
         std::uint32_t const m = find_mesh(begin, mesh_count, i);
-        refit_moments_item<Order>(meshes[m], i - begin[m]);
+        refit_moments_item<Order>(meshes[m], i - begin[m], s_even + threadIdx.x);
     }
 }
 
