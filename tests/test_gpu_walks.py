@@ -1,0 +1,93 @@
+"""Walks that change form on the way: small batches, warp walks given up for the lanes' own (Taylor and
+distance), and distance queries left to the one-query-per-warp kernel. Every form takes the same decisions,
+sums in the same order (Taylor) or takes a minimum (distance), so results are equal bit for bit to those of
+the walk of one query per thread."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import oracle
+import smallgwn_b200 as g
+from smallgwn_b200 import api, meshes
+from test_gpu_build import build, upload
+from test_gpu_query import dev, moments_of
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def scene():
+    mesh = meshes.to_soa(*meshes.uv_sphere(256, 128, 7))
+    geo = upload(mesh)
+    bvh = build(geo, g.gwn_bvh_build_method.k_hploc)
+    return mesh, geo, bvh, {o: moments_of(bvh, o) for o in (0, 1, 2)}
+
+
+def taylor(cuda, order, bvh, mom, d, traversal, precision, sort=True):
+    out = cuda.full_like(d[0], float("nan"))
+    st = g.gwn_compute_winding_number_taylor_batch(order, bvh, mom, *d, out, precision=precision, traversal=traversal,
+                                                   sort_queries=sort)
+    assert st.is_ok(), st.message
+    return out.cpu().numpy()
+
+
+# around the batch sizes at which the queries per warp change (32 warps per SM), and sparse large ones
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 1000, 4736, 4737, 9473, 75777, 200_003])
+@pytest.mark.parametrize("order,precision", [(0, 0), (1, 1), (2, 0), (2, 1)])
+def test_taylor_walks_agree(cuda, scene, n, order, precision):
+    mesh, _, bvh, moms = scene
+    mixes = (meshes.mixed_queries(mesh, n, seed=n), meshes.reference_mixed_queries(mesh, n, seed=n))
+    for q in mixes if n < 100_000 else mixes[1:]:
+        d = dev(cuda, *q)
+        ref = taylor(cuda, order, bvh, moms[order], d, "thread", precision)
+        assert np.isfinite(ref).all()
+        for sort in (True, False):
+            np.testing.assert_array_equal(taylor(cuda, order, bvh, moms[order], d, "warp", precision, sort), ref)
+
+
+@pytest.mark.parametrize("n", [5, 4737, 100_001])
+@pytest.mark.parametrize("order", [1, 2])
+def test_gradient_walks_agree(cuda, scene, n, order):
+    mesh, _, bvh, moms = scene
+    d = dev(cuda, *meshes.reference_mixed_queries(mesh, n, seed=n))
+    res = []
+    for traversal in ("warp", "thread"):
+        gs = [cuda.full_like(d[0], float("nan")) for _ in range(3)]
+        st = g.gwn_compute_winding_gradient_taylor_batch(order, bvh, moms[order], *d, *gs, traversal=traversal)
+        assert st.is_ok(), st.message
+        res.append(np.stack([x.cpu().numpy() for x in gs]))
+    np.testing.assert_array_equal(res[0], res[1])
+
+
+@pytest.mark.parametrize("n", [1, 33, 4736, 4737, 30_001])
+@pytest.mark.parametrize("band", [float("inf"), 0.9, 0.0])
+def test_distance_walks_agree(cuda, n, band):
+    """A round sphere and queries around its centre, from which most of the surface is equally far: every
+    walk is given up; beside them queries on vertices, outside, far away and not a number."""
+    mesh = meshes.to_soa(*meshes.uv_sphere(160, 80, 0, displaced=False))
+    bvh = build(upload(mesh), g.gwn_bvh_build_method.k_hploc)
+    rng = np.random.default_rng(n)
+    q = np.concatenate([rng.normal(0, 0.02, (3, n - n // 2)), rng.uniform(-2, 2, (3, n // 2))], 1).astype(np.float32)
+    if n > 30:
+        q[:, 5] = [mesh[k][100] for k in "xyz"]
+        q[:, 6] = np.nan
+        q[:, 7] = 1e6
+    d = dev(cuda, *q)
+
+    def run(**kw):
+        out = cuda.full_like(d[0], float("nan"))
+        st = g.gwn_compute_unsigned_distance_batch(bvh, *d, out, culling_band=band, **kw)
+        assert st.is_ok(), st.message
+        return out.cpu().numpy()
+
+    ref = run(sort_queries=True, traversal="thread")
+    np.testing.assert_array_equal(run(sort_queries=True), ref)
+    np.testing.assert_array_equal(run(sort_queries=False), ref)
+    h = api.bvh_host_arrays(bvh)
+    some = slice(0, min(n, 2000))
+    want = oracle.mesh_distance(mesh, *q[:, some])
+    ok = np.isfinite(want) & (want < 10)
+    # 2e-6: test_gpu_spatial's bound against FP64 closest points
+    assert np.abs(ref[some][ok] - np.minimum(want[ok], band)).max(initial=0.0) <= 2e-6
+    assert h["internal_stack_bound"] <= 64
