@@ -58,6 +58,11 @@ struct spatial_params {
     int stack_cap; // entries of this thread's stack column (the BVH's internal stack bound, at least 1)
     unsigned int *status;
     unsigned long long *next_item; // persistent kernels: first unclaimed sorted position (zeroed per launch)
+    // distance batches: queries given up after a number of nodes (their squared bound waits in distance[]),
+    // finished by k_distance_long; nullptr: none are given up
+    std::uint32_t *long_items;
+    unsigned int *long_count;
+    unsigned int *long_next; // first unclaimed entry
 };
 
 // ---- arithmetic: every product, sum and quotient rounded on its own, fused multiply-adds in one
@@ -204,12 +209,22 @@ __device__ __forceinline__ float point_triangle_d2(v3 p, v3 a, v3 b, v3 c) {
     return dot(q, q);
 }
 
+// Nodes after which a query's own walk, and a warp's union walk, is given up to k_distance_long. A
+// query near the middle of a round mesh has most of the surface at about its distance: on the 1M-triangle
+// sphere the mean is 240 nodes, the longest query takes 9,600, and a batch of 2M ended 30 ms after the
+// work of all other warps. 2M ordered / 500k unordered / 50k ordered queries: 54.9 / 20.0 / 10.0 ms without,
+// 26.4 / 8.3 / 1.7 ms with 128 and 512 nodes, 26.8 / 10.2 / 2.7 with 256 and 1,024, 29.9 / 13.4 / 6.5 with
+// 1,024 and 4,096.
+constexpr int k_alone_nodes = 128;
+constexpr int k_union_nodes = 512;
+
 // The state of one distance query between node visits (see ray_lane).
 struct distance_lane {
     v3 q;
     float best; // squared distance bound
     std::uint32_t qi, node, st_nodes, st_tris;
     int sp;
+    int left;     // nodes until the query is given up (k_distance_walk)
     bool touched; // a triangle touches the query: distance 0 is final
 };
 
@@ -233,14 +248,19 @@ __device__ __forceinline__ void distance_leaf(spatial_params const &p, distance_
     L.touched = !(L.best > 0.0f);
 }
 
+// A thread's column of a [p.stack_cap][blockDim.x] shared-memory stack.
+struct stack_column {
+    std::uint32_t *p;
+    __device__ __forceinline__ std::uint32_t &operator()(int e) const { return p[static_cast<unsigned>(e) * blockDim.x]; }
+};
+
 // One node of detail/gwn_query_distance_impl.cuh:40-160 for L.node: children within the bound
 // sorted near first, leaf children inside the node, internal children far to near with the
-// nearest entered directly. s_stack is this thread's column of a [p.stack_cap][blockDim.x]
-// shared-memory stack of internal node indices. False once the query is finished.
-template <bool Stats>
-__device__ __forceinline__ bool distance_visit(spatial_params const &p, distance_lane &L, std::uint32_t *s_stack,
+// nearest entered directly. stack is an indexable column of p.stack_cap internal node indices.
+// False once the query is finished.
+template <bool Stats, class Stack>
+__device__ __forceinline__ bool distance_visit(spatial_params const &p, distance_lane &L, Stack &&stack,
                                                bool &overflow) {
-    unsigned const stride = blockDim.x;
     if constexpr (Stats)
         ++L.st_nodes;
     float4 const *nd = p.nodes + static_cast<std::uint64_t>(L.node) * 8;
@@ -279,7 +299,7 @@ __device__ __forceinline__ bool distance_visit(spatial_params const &p, distance
                 overflow = true;
                 continue;
             }
-            s_stack[static_cast<unsigned>(L.sp) * stride] = next;
+            stack(L.sp) = next;
             ++L.sp;
         }
         next = v;
@@ -293,7 +313,7 @@ __device__ __forceinline__ bool distance_visit(spatial_params const &p, distance
     if (L.sp == 0)
         return false;
     --L.sp;
-    L.node = s_stack[static_cast<unsigned>(L.sp) * stride];
+    L.node = stack(L.sp);
     return true;
 }
 
@@ -308,6 +328,7 @@ __device__ __forceinline__ bool distance_begin(spatial_params const &p, std::uin
     L.st_nodes = 0;
     L.st_tris = 0;
     L.sp = 0;
+    L.left = k_alone_nodes;
     L.touched = false;
     if (ref_leaf(p.root_ref)) {
         distance_leaf<Stats>(p, L, p.root_ref);
@@ -317,6 +338,12 @@ __device__ __forceinline__ bool distance_begin(spatial_params const &p, std::uin
         return false;
     L.node = static_cast<std::uint32_t>(ref_offset(p.root_ref));
     return true;
+}
+
+// Hands an unfinished query to k_distance_long.
+__device__ __forceinline__ void distance_defer(spatial_params const &p, distance_lane const &L) {
+    p.distance[L.qi] = L.best;
+    p.long_items[atomicAdd(p.long_count, 1u)] = L.qi;
 }
 
 template <bool Stats>
@@ -610,6 +637,7 @@ struct ray_walk {
     static __device__ __forceinline__ bool step(spatial_params const &p, lane &L, std::uint32_t *col, bool &overflow) {
         return ray_step<Stats>(p, L, col, overflow);
     }
+    template <bool Stats> static __device__ __forceinline__ bool give_up(spatial_params const &, lane &) { return false; }
     template <bool Stats> static __device__ __forceinline__ void finish(spatial_params const &p, lane const &L, bool o) {
         ray_finish<Stats>(p, L, o);
     }
@@ -622,7 +650,14 @@ struct distance_walk {
     }
     template <bool Stats>
     static __device__ __forceinline__ bool step(spatial_params const &p, lane &L, std::uint32_t *col, bool &overflow) {
-        return distance_visit<Stats>(p, L, col, overflow);
+        return distance_visit<Stats>(p, L, stack_column{col}, overflow);
+    }
+    // a query of very many nodes is left to k_distance_long
+    template <bool Stats> static __device__ __forceinline__ bool give_up(spatial_params const &p, lane &L) {
+        if (Stats || p.long_items == nullptr || --L.left > 0)
+            return false;
+        distance_defer(p, L);
+        return true;
     }
     template <bool Stats> static __device__ __forceinline__ void finish(spatial_params const &p, lane const &L, bool o) {
         distance_finish<Stats>(p, L, o);
@@ -672,9 +707,13 @@ template <class W, bool Stats> __device__ __forceinline__ void walk(spatial_para
         }
         if (__ballot_sync(0xffffffffu, have) == 0u)
             break;
-        if (have && !W::template step<Stats>(p, L, col, overflow)) {
-            W::template finish<Stats>(p, L, overflow);
-            have = false;
+        if (have) {
+            if (!W::template step<Stats>(p, L, col, overflow)) {
+                W::template finish<Stats>(p, L, overflow);
+                have = false;
+            } else if (W::template give_up<Stats>(p, L)) {
+                have = false;
+            }
         }
     }
 }
@@ -685,7 +724,12 @@ template <bool Stats> __global__ void __launch_bounds__(256) k_ray(spatial_param
     walk<ray_walk, Stats>(p, s_stack + threadIdx.x);
 }
 
-// Distance queries in Hilbert order stay one per thread: a warp's traversals are similar enough
+// The union walk is left for the lanes' own walks as the Taylor walk is: every node taken from the stack
+// earns the lanes that need it and costs this many.
+constexpr int k_union_lanes = 8;
+constexpr int k_union_credit = 64;
+
+// Distance queries in Hilbert order stay one per thread here: a warp's traversals are similar enough
 // that refilling lanes costs as much coherence as it saves (10M queries on the 1M-triangle sphere:
 // 96 ms one per thread, 100 ms persistent). Queries in input order take the persistent form
 // (k_distance_walk: 104 ms against 291 ms one per thread).
@@ -697,7 +741,7 @@ template <bool Stats> __global__ void __launch_bounds__(256) k_distance(spatial_
     distance_lane L;
     bool overflow = false;
     if (distance_begin<Stats>(p, idx, L))
-        while (distance_visit<Stats>(p, L, s_stack + threadIdx.x, overflow)) {
+        while (distance_visit<Stats>(p, L, stack_column{s_stack + threadIdx.x}, overflow)) {
         }
     distance_finish<Stats>(p, L, overflow);
 }
@@ -713,7 +757,9 @@ template <bool Stats> __global__ void __launch_bounds__(256) k_distance(spatial_
 // the same minimum -- only the order of the visits differs (and with it how soon a bound tightens).
 // The stack lives in the lanes' registers (entry e in lane e & 31, bank e >> 5), as in the Taylor
 // warp walk; the union walk never holds more entries than the tree's internal stack bound.
-template <int Cap> __global__ void __launch_bounds__(256) k_distance_warp(spatial_params p) {
+// A warp whose lanes share too little of what is left goes on lane by lane (k_union_lanes), and what
+// either form has not finished after its number of nodes is left to k_distance_long.
+template <int Cap> __global__ void __launch_bounds__(256, 4) k_distance_warp(spatial_params p) {
     static_assert(Cap <= 64, "warp stack holds at most 64 entries");
     unsigned const lane = threadIdx.x & 31u;
     std::uint64_t const idx = static_cast<std::uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -729,7 +775,11 @@ template <int Cap> __global__ void __launch_bounds__(256) k_distance_warp(spatia
         std::uint32_t st_node0 = 0, st_node1 = 0;
         unsigned st_mask0 = 0, st_mask1 = 0;
         int sp = 0;
+        int credit = k_union_credit; // negative: the walk is given up
+        int left = k_union_nodes;
         for (;;) {
+            if (credit < 0 || --left < 0)
+                break;
             mask &= __ballot_sync(0xffffffffu, walks && !L.touched);
             if (mask != 0u && node < p.node_count) {
                 bool const active = ((mask >> lane) & 1u) != 0u;
@@ -835,10 +885,149 @@ template <int Cap> __global__ void __launch_bounds__(256) k_distance_warp(spatia
                 node = __shfl_sync(0xffffffffu, st_node1, src);
                 mask = __shfl_sync(0xffffffffu, st_mask1, src);
             }
+            credit += __popc(mask) - k_union_lanes;
+        }
+        if (!overflow && (credit < 0 || left < 0)) {
+            // each lane's share of the stack, and its walk from there
+            std::uint32_t own[Cap];
+            L.sp = 0;
+            for (int e = 0; e < sp; ++e) {
+                std::uint32_t const n = __shfl_sync(0xffffffffu, e < 32 ? st_node0 : st_node1, e & 31);
+                unsigned const m = __shfl_sync(0xffffffffu, e < 32 ? st_mask0 : st_mask1, e & 31);
+                if (((m >> lane) & 1u) != 0u)
+                    own[L.sp++] = n;
+            }
+            bool const here = ((mask >> lane) & 1u) != 0u;
+            bool more = walks && !L.touched && (here || L.sp > 0);
+            L.node = here || L.sp == 0 ? node : own[--L.sp];
+            for (int k = left < 0 ? 0 : k_alone_nodes; more && k > 0; --k)
+                more = L.node < p.node_count &&
+                       distance_visit<false>(p, L, [&](int e) -> std::uint32_t & { return own[e]; }, overflow);
+            if (more) {
+                distance_defer(p, L);
+                return;
+            }
         }
     }
     if (valid)
         distance_finish<false>(p, L, walks && overflow);
+}
+
+// One query per warp: the queries k_distance_warp gave up, or all of a batch too small to fill the GPU
+// (long_items == nullptr). The lanes take the warp's 32 uppermost stack entries at a time (node and box
+// distance, in shared memory), test their children against the warp's common bound, evaluate the leaf
+// children and push the internal ones, nearest uppermost, so that a query of thousands of nodes takes
+// some hundred steps. A minimum does not depend on the order of the triangles, so the result is the same.
+constexpr int k_long_block = 256;
+constexpr int k_long_stack = 512; // entries per warp
+
+__global__ void __launch_bounds__(k_long_block) k_distance_long(spatial_params p) {
+    __shared__ std::uint32_t s_node[k_long_block / 32][k_long_stack];
+    __shared__ float s_key[k_long_block / 32][k_long_stack];
+    constexpr unsigned all = 0xffffffffu;
+    unsigned const lane = threadIdx.x & 31u;
+    std::uint32_t *const nodes = s_node[threadIdx.x >> 5];
+    float *const keys = s_key[threadIdx.x >> 5];
+    unsigned const total = p.long_items != nullptr ? *p.long_count : static_cast<unsigned>(p.n);
+    for (;;) {
+        unsigned item = 0;
+        if (lane == 0)
+            item = atomicAdd(p.long_next, 1u);
+        item = __shfl_sync(all, item, 0);
+        if (item >= total)
+            return;
+        distance_lane L;
+        bool walks;
+        if (p.long_items != nullptr) {
+            L.qi = p.long_items[item];
+            L.q = v3{p.qx[L.qi], p.qy[L.qi], p.qz[L.qi]};
+            L.best = p.distance[L.qi];
+            L.touched = false;
+            L.node = static_cast<std::uint32_t>(ref_offset(p.root_ref));
+            walks = true;
+        } else {
+            walks = distance_begin<false>(p, item, L);
+        }
+        bool overflow = false;
+        int sp = 0;
+        if (walks) {
+            if (lane == 0) {
+                nodes[0] = L.node;
+                keys[0] = -1.0f; // the root is entered whatever its distance
+            }
+            sp = 1;
+            __syncwarp();
+        }
+        // above this height only one entry is taken at a time: a depth-first walk from there adds at
+        // most the tree's stack bound and the last node's children
+        int const high = k_long_stack - p.stack_cap - 4;
+        while (sp > 0) {
+            int n = sp < 32 ? sp : 32;
+            if (sp + 3 * n > high)
+                n = sp < high - 3 ? (high - sp) / 3 : 1;
+            bool const take = static_cast<int>(lane) < n;
+            std::uint32_t const node = take ? nodes[sp - 1 - static_cast<int>(lane)] : 0u;
+            float const key = take ? keys[sp - 1 - static_cast<int>(lane)] : 0.0f;
+            sp -= n;
+            __syncwarp();
+            cand4 cd;
+            int cnt = 0;
+            if (take && key < L.best && node < p.node_count) {
+                float4 const *nd = p.nodes + static_cast<std::uint64_t>(node) * 8;
+#pragma unroll
+                for (int s = 0; s < 4; ++s) {
+                    float4 const A = __ldg(nd + 2 * s);
+                    float4 const B = __ldg(nd + 2 * s + 1);
+                    std::uint64_t const ref = (static_cast<std::uint64_t>(__float_as_uint(B.w)) << 32) | __float_as_uint(B.z);
+                    if (!ref_valid(ref))
+                        continue;
+                    float const d2 = aabb_d2(L.q, A, B);
+                    if (!(d2 < L.best))
+                        continue;
+                    if (ref_leaf(ref)) {
+                        distance_leaf<false>(p, L, ref);
+                    } else if (ref_offset(ref) < p.node_count) {
+                        cd.put(cnt, d2, static_cast<std::uint32_t>(ref_offset(ref)));
+                        ++cnt;
+                    }
+                }
+            }
+            // squared distances are not negative, so their bits order like the values
+            L.best = __uint_as_float(__reduce_min_sync(all, __float_as_uint(L.best)));
+            L.touched = __any_sync(all, L.touched);
+            if (L.touched)
+                break;
+            cd.sort(cnt);
+            int keep = 0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                keep += k < cnt && cd.key[k] < L.best ? 1 : 0;
+            // lane 0 took the uppermost entry: its children go on top, each lane's nearest above its others
+            int below = keep; // entries of this lane and of those after it
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                int const v = __shfl_down_sync(all, below, d);
+                below += lane + static_cast<unsigned>(d) < 32u ? v : 0;
+            }
+            int const added = __shfl_sync(all, below, 0);
+            if (sp + added > k_long_stack) {
+                overflow = true;
+                break;
+            }
+            int const at = sp + below - 1; // this lane's uppermost entry
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (k < keep) {
+                    nodes[at - k] = cd.pay[k];
+                    keys[at - k] = cd.key[k];
+                }
+            sp += added;
+            __syncwarp();
+        }
+        __syncwarp();
+        if (lane == 0)
+            distance_finish<false>(p, L, overflow);
+    }
 }
 
 template <bool Stats> __global__ void __launch_bounds__(256) k_distance_walk(spatial_params p) {
@@ -934,6 +1123,49 @@ template <class Kern> int launch_persistent(Kern kern, spatial_params p, int blo
     return GWNB_OK;
 }
 
+// One query per warp: those listed in p.long_items, or all n.
+int launch_distance_long(spatial_params const &p, cudaStream_t s) {
+    std::uint64_t const warps = k_long_block / 32;
+    std::uint64_t const resident = static_cast<std::uint64_t>(device_sm_count()) * 4;
+    std::uint64_t const needed = (p.n + warps - 1) / warps;
+    note_launch(), k_distance_long<<<static_cast<unsigned>(needed < resident ? needed : resident), k_long_block, 0, s>>>(p);
+    GWNB_CUDA_TRY(cudaGetLastError());
+    return GWNB_OK;
+}
+
+// Batches that fill less than this many warps per SM with one query each take k_distance_long alone.
+constexpr std::uint64_t k_long_alone_warps = 32;
+
+int launch_distance_few(spatial_params p, cudaStream_t s) {
+    unsigned int *next = nullptr;
+    GWNB_TRY(alloc(&next, 1, s));
+    p.long_next = next;
+    int rc = GWNB_OK;
+    cudaError_t const e = cudaMemsetAsync(next, 0, sizeof(unsigned int), s);
+    if (e != cudaSuccess)
+        rc = set_cuda_error(e, "distance batch counter");
+    if (rc == GWNB_OK)
+        rc = launch_distance_long(p, s);
+    release(next, s);
+    return rc;
+}
+
+// A distance kernel that may give queries up (`launch`, handed the parameters with the list), and after it
+// the queries that it did.
+template <class F> int launch_distance_deferring(spatial_params p, cudaStream_t s, F &&launch) {
+    std::uint32_t *items = nullptr; // [n] queries given up, then their count and the next to claim
+    GWNB_TRY(alloc(&items, p.n + 2, s));
+    p.long_items = items;
+    p.long_count = items + p.n;
+    p.long_next = items + p.n + 1;
+    cudaError_t const e = cudaMemsetAsync(p.long_count, 0, 2 * sizeof(unsigned int), s);
+    int rc = e == cudaSuccess ? launch(p) : set_cuda_error(e, "distance batch counters");
+    if (rc == GWNB_OK)
+        rc = launch_distance_long(p, s);
+    release(items, s);
+    return rc;
+}
+
 template <int Cap> int launch_distance_warp(spatial_params const &p, cudaStream_t s) {
     unsigned const grid = static_cast<unsigned>((p.n + 255) / 256);
     note_launch(), k_distance_warp<Cap><<<grid, 256, 0, s>>>(p);
@@ -946,7 +1178,12 @@ template <bool Ray, bool Stats> int launch_spatial(spatial_params const &p, int 
     if (Ray)
         return launch_persistent(k_ray<Stats>, p, block, s);
     if (warp_walk)
-        return p.stack_cap <= 32 ? launch_distance_warp<32>(p, s) : launch_distance_warp<64>(p, s);
+        return launch_distance_deferring(p, s, [&](spatial_params const &q) {
+            return q.stack_cap <= 32 ? launch_distance_warp<32>(q, s) : launch_distance_warp<64>(q, s);
+        });
+    if (p.order == nullptr && !Stats && p.stack_cap <= k_long_stack / 2)
+        return launch_distance_deferring(
+            p, s, [&](spatial_params const &q) { return launch_persistent(k_distance_walk<Stats>, q, block, s); });
     return p.order != nullptr ? launch_per_query(k_distance<Stats>, p, block, s)
                               : launch_persistent(k_distance_walk<Stats>, p, block, s);
 }
@@ -1009,7 +1246,10 @@ int spatial_batch(gwnb_bvh4_f32 *b, spatial_request const &r, cudaStream_t s) {
     p.t_max = r.t_max;
     p.status = a->status;
     std::uint32_t *order = nullptr;
-    if (r.opt.sort_queries != 0 && r.n > 1) {
+    // a small distance batch takes one query per warp, in any order
+    bool const few = !r.ray && r.stat_nodes == nullptr && r.opt.per_thread == GWNB_WALK_WARP &&
+                     r.n <= static_cast<std::uint64_t>(device_sm_count()) * k_long_alone_warps;
+    if (r.opt.sort_queries != 0 && r.n > 1 && !few) {
         GWNB_TRY(alloc(&order, r.n, s));
         int const rc = r.ray ? ray_order(a, r.qx, r.qy, r.qz, r.dx, r.dy, r.dz, r.n, order, s)
                              : query_order(a->root_bounds, r.qx, r.qy, r.qz, r.n, order, s, a->status);
@@ -1024,6 +1264,8 @@ int spatial_batch(gwnb_bvh4_f32 *b, spatial_request const &r, cudaStream_t s) {
     if (p.stack_cap < 1)
         p.stack_cap = 1;
     bool const stats = r.stat_nodes != nullptr;
+    if (few && p.stack_cap <= k_long_stack / 2)
+        return launch_distance_few(p, s);
     // the walk of a distance batch in Hilbert order (the statistics keep the per-thread walk, whose
     // visit counts are the canonical traversal's)
     walk_plan plan;
