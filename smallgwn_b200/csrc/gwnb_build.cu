@@ -319,6 +319,163 @@ __device__ std::uint32_t collapse_tile_prefix(unsigned long long *st, std::uint3
     return excl;
 }
 
+// What the threads of a tile know between choosing their children and writing their node.
+struct collapse_choice {
+    std::uint32_t cidx[4], ckind[4];
+    int k = 0; // children
+    std::uint32_t internal = 0;
+    collapse_item item{0, 0, 0};
+};
+
+// The (up to four) children of item i of a level: every index into cidx / ckind is a compile-time
+// constant, so both stay in registers.
+__device__ __forceinline__ collapse_choice collapse_choose(collapse_params const &p, collapse_item const *items_in,
+                                                           std::uint32_t i, bool valid) {
+    collapse_choice r;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+        r.cidx[c] = r.ckind[c] = 0;
+    if (!valid)
+        return r;
+    r.item = items_in[i];
+    if (r.item.binary_index >= p.leaf_count - 1) {
+        atomicOr(p.status, k_err_collapse);
+        return r;
+    }
+    binary_node const root = p.binary[r.item.binary_index];
+    r.cidx[0] = root.left_index;
+    r.ckind[0] = root.left_kind;
+    r.cidx[1] = root.right_index;
+    r.ckind[1] = root.right_kind;
+    r.k = 2;
+    // Expand the largest-area internal child (ties: smallest binary index) until four children or only
+    // leaves remain.
+#pragma unroll
+    for (int step = 0; step < 2; ++step) {
+        int best = -1;
+        float best_area = -__int_as_float(0x7f800000);
+        std::uint32_t best_index = k_invalid_u32;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (c >= r.k || r.ckind[c] != k_kind_internal || r.cidx[c] >= p.leaf_count - 1)
+                continue;
+            float const area = aabb_half_area(p.binary_bounds[r.cidx[c]]);
+            if (best >= 0 && area < best_area)
+                continue;
+            if (best >= 0 && area == best_area && r.cidx[c] >= best_index)
+                continue;
+            best = c;
+            best_area = area;
+            best_index = r.cidx[c];
+        }
+        if (best < 0)
+            break;
+        binary_node const e = p.binary[best_index];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (c == best) {
+                r.cidx[c] = e.left_index;
+                r.ckind[c] = e.left_kind;
+            } else if (c == r.k) {
+                r.cidx[c] = e.right_index;
+                r.ckind[c] = e.right_kind;
+            }
+        }
+        ++r.k;
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+        r.internal += (c < r.k && r.ckind[c] == k_kind_internal) ? 1u : 0u;
+    return r;
+}
+
+// Exclusive sum of the threads' internal-child counts over a block of Block threads, and their total.
+// s_scan holds one word per warp; a barrier must separate two uses.
+template <int Block>
+__device__ __forceinline__ std::uint32_t collapse_scan(std::uint32_t v, std::uint32_t *s_scan, std::uint32_t &total) {
+    unsigned const lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    std::uint32_t incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        std::uint32_t const t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= static_cast<unsigned>(o))
+            incl += t;
+    }
+    if (lane == 31)
+        s_scan[warp] = incl;
+    __syncthreads();
+    std::uint32_t prefix = 0;
+    total = 0;
+    for (int w = 0; w < Block / 32; ++w) {
+        if (static_cast<unsigned>(w) < warp)
+            prefix += s_scan[w];
+        total += s_scan[w];
+    }
+    return prefix + incl - v;
+}
+
+// Writes the node of item i of the level (n_in items from node index `base`), its internal children being
+// the next level's items from out_first on.
+__device__ __forceinline__ void collapse_write(collapse_params const &p, collapse_choice const &r, std::uint32_t i,
+                                               std::uint32_t n_in, std::uint32_t base, std::uint32_t out_first,
+                                               collapse_item *items_out) {
+    std::uint32_t const w = base + i;
+    std::uint32_t const id_first = base + n_in + out_first;
+    std::uint32_t const node_int = r.item.prefix_internal + (r.internal > 0 ? r.internal - 1u : 0u);
+    std::uint32_t const node_pk = r.item.prefix_packed + static_cast<std::uint32_t>(r.k - 1);
+    // only a broken binary hierarchy can produce more items than the list holds
+    bool const room = static_cast<std::uint64_t>(out_first) + r.internal <= p.list_capacity;
+    if (!room)
+        atomicOr(p.status, k_err_collapse);
+    bool const node_ok = w < p.node_capacity;
+    if (!node_ok)
+        atomicOr(p.status, k_err_collapse);
+    float4 *const dst = reinterpret_cast<float4 *>(p.nodes + (node_ok ? w : 0u));
+    std::uint32_t m = 0;
+    // Each child is written as two 16-byte stores straight from registers.
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        aabb bb{0, 0, 0, 0, 0, 0};
+        std::uint64_t ref = 0;
+        if (c < r.k) {
+            if (r.ckind[c] == k_kind_leaf) {
+                if (r.cidx[c] < p.leaf_count) {
+                    bb = p.leaf_aabbs[r.cidx[c]];
+                    ref = make_ref(r.cidx[c], 1u);
+                } else {
+                    atomicOr(p.status, k_err_collapse);
+                }
+            } else {
+                if (r.cidx[c] < p.leaf_count - 1)
+                    bb = p.binary_bounds[r.cidx[c]];
+                else
+                    atomicOr(p.status, k_err_collapse);
+                ref = make_ref(id_first + m, 0u);
+                if (room)
+                    items_out[out_first + m] = collapse_item{r.cidx[c], node_int, node_pk};
+                ++m;
+            }
+        }
+        if (node_ok) {
+            dst[2 * c] = make_float4(bb.min_x, bb.min_y, bb.min_z, bb.max_x);
+            dst[2 * c + 1] = make_float4(bb.max_y, bb.max_z, __uint_as_float(static_cast<std::uint32_t>(ref)),
+                                         __uint_as_float(static_cast<std::uint32_t>(ref >> 32)));
+        }
+    }
+    atomicMax(&p.stack_bounds[0], node_int);
+    atomicMax(&p.stack_bounds[1], node_pk);
+}
+
+// Items of a level, checked: only a broken binary hierarchy can hold more than internal nodes.
+__device__ __forceinline__ std::uint32_t collapse_level_items(collapse_params const &p, int level) {
+    std::uint32_t const n = *reinterpret_cast<volatile std::uint32_t *>(&p.level_count[level]);
+    if (n <= p.list_capacity)
+        return n;
+    if (threadIdx.x == 0)
+        atomicOr(p.status, k_err_collapse);
+    return 0;
+}
+
 // One level of the collapse: blocks claim tiles of k_block items from the level's counter in launch
 // order (so a tile's look-back only ever waits on tiles claimed before it) until the level is
 // exhausted.
@@ -326,21 +483,13 @@ __global__ void __launch_bounds__(k_block) k_collapse_level(collapse_params p, i
     __shared__ std::uint32_t s_tile;
     __shared__ std::uint32_t s_prefix;
     __shared__ std::uint32_t s_scan[k_block / 32];
-    std::uint32_t n_in = *reinterpret_cast<volatile std::uint32_t *>(&p.level_count[level]);
-    if (n_in > p.list_capacity) {
-        // only a broken binary hierarchy can hold more items on one level than internal nodes
-        if (threadIdx.x == 0)
-            atomicOr(p.status, k_err_collapse);
-        n_in = 0;
-    }
+    std::uint32_t const n_in = collapse_level_items(p, level);
     std::uint32_t const base = *reinterpret_cast<volatile std::uint32_t *>(&p.level_base[level]);
     // selected, not indexed: a run-time index into the parameter array would copy it to local memory
     bool const odd = (level & 1) != 0;
     collapse_item const *items_in = odd ? p.lists[1] : p.lists[0];
     collapse_item *items_out = odd ? p.lists[0] : p.lists[1];
     unsigned const tid = threadIdx.x;
-    unsigned const lane = tid & 31u;
-    unsigned const warp = tid >> 5;
     unsigned long long const tag = static_cast<unsigned long long>(level + 1) << 34;
 
     for (;;) {
@@ -353,83 +502,9 @@ __global__ void __launch_bounds__(k_block) k_collapse_level(collapse_params p, i
             break;
         std::uint32_t const i = tile * k_block + tid;
         bool const valid = i < n_in;
-
-        std::uint32_t cidx[4] = {0, 0, 0, 0};
-        std::uint32_t ckind[4] = {0, 0, 0, 0};
-        int k = 0;
-        std::uint32_t k_int = 0;
-        collapse_item item{0, 0, 0};
-        if (valid) {
-            item = items_in[i];
-            if (item.binary_index >= p.leaf_count - 1) {
-                atomicOr(p.status, k_err_collapse);
-            } else {
-                binary_node const root = p.binary[item.binary_index];
-                cidx[0] = root.left_index;
-                ckind[0] = root.left_kind;
-                cidx[1] = root.right_index;
-                ckind[1] = root.right_kind;
-                k = 2;
-                // Expand the largest-area internal child (ties: smallest binary index) until four
-                // children or only leaves remain; every index into cidx/ckind is a compile-time
-                // constant, so both stay in registers.
-#pragma unroll
-                for (int step = 0; step < 2; ++step) {
-                    int best = -1;
-                    float best_area = -__int_as_float(0x7f800000);
-                    std::uint32_t best_index = k_invalid_u32;
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        if (c >= k || ckind[c] != k_kind_internal || cidx[c] >= p.leaf_count - 1)
-                            continue;
-                        float const area = aabb_half_area(p.binary_bounds[cidx[c]]);
-                        if (best >= 0 && area < best_area)
-                            continue;
-                        if (best >= 0 && area == best_area && cidx[c] >= best_index)
-                            continue;
-                        best = c;
-                        best_area = area;
-                        best_index = cidx[c];
-                    }
-                    if (best < 0)
-                        break;
-                    binary_node const e = p.binary[best_index];
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        if (c == best) {
-                            cidx[c] = e.left_index;
-                            ckind[c] = e.left_kind;
-                        } else if (c == k) {
-                            cidx[c] = e.right_index;
-                            ckind[c] = e.right_kind;
-                        }
-                    }
-                    ++k;
-                }
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    k_int += (c < k && ckind[c] == k_kind_internal) ? 1u : 0u;
-            }
-        }
-
-        // Block scan of internal-child counts.
-        std::uint32_t incl = k_int;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            std::uint32_t const t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= static_cast<unsigned>(o))
-                incl += t;
-        }
-        if (lane == 31)
-            s_scan[warp] = incl;
-        __syncthreads();
-        std::uint32_t warp_prefix = 0, block_total = 0;
-        for (int w = 0; w < k_block / 32; ++w) {
-            if (static_cast<unsigned>(w) < warp)
-                warp_prefix += s_scan[w];
-            block_total += s_scan[w];
-        }
-        std::uint32_t const local_excl = warp_prefix + incl - k_int;
+        collapse_choice const r = collapse_choose(p, items_in, i, valid);
+        std::uint32_t block_total;
+        std::uint32_t const local_excl = collapse_scan<k_block>(r.internal, s_scan, block_total);
 
         // Decoupled look-back over tiles of this level.
         if (tid == 0)
@@ -438,58 +513,53 @@ __global__ void __launch_bounds__(k_block) k_collapse_level(collapse_params p, i
         std::uint32_t const tile_prefix = s_prefix;
         __syncthreads();
 
-        if (valid && k > 0) {
-            std::uint32_t const w = base + i;
-            std::uint32_t const out_first = tile_prefix + local_excl;
-            std::uint32_t const id_first = base + n_in + out_first;
-            std::uint32_t const node_int = item.prefix_internal + (k_int > 0 ? k_int - 1u : 0u);
-            std::uint32_t const node_pk = item.prefix_packed + static_cast<std::uint32_t>(k - 1);
-            // only a broken binary hierarchy can produce more items than the list holds
-            bool const room = static_cast<std::uint64_t>(out_first) + k_int <= p.list_capacity;
-            if (!room)
-                atomicOr(p.status, k_err_collapse);
-            bool const node_ok = w < p.node_capacity;
-            if (!node_ok)
-                atomicOr(p.status, k_err_collapse);
-            float4 *const dst = reinterpret_cast<float4 *>(p.nodes + (node_ok ? w : 0u));
-            std::uint32_t m = 0;
-            // Each child is written as two 16-byte stores straight from registers.
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                aabb bb{0, 0, 0, 0, 0, 0};
-                std::uint64_t ref = 0;
-                if (c < k) {
-                    if (ckind[c] == k_kind_leaf) {
-                        if (cidx[c] < p.leaf_count) {
-                            bb = p.leaf_aabbs[cidx[c]];
-                            ref = make_ref(cidx[c], 1u);
-                        } else {
-                            atomicOr(p.status, k_err_collapse);
-                        }
-                    } else {
-                        if (cidx[c] < p.leaf_count - 1)
-                            bb = p.binary_bounds[cidx[c]];
-                        else
-                            atomicOr(p.status, k_err_collapse);
-                        ref = make_ref(id_first + m, 0u);
-                        if (room)
-                            items_out[out_first + m] = collapse_item{cidx[c], node_int, node_pk};
-                        ++m;
-                    }
-                }
-                if (node_ok) {
-                    dst[2 * c] = make_float4(bb.min_x, bb.min_y, bb.min_z, bb.max_x);
-                    dst[2 * c + 1] = make_float4(bb.max_y, bb.max_z, __uint_as_float(static_cast<std::uint32_t>(ref)),
-                                                 __uint_as_float(static_cast<std::uint32_t>(ref >> 32)));
-                }
-            }
-            atomicMax(&p.stack_bounds[0], node_int);
-            atomicMax(&p.stack_bounds[1], node_pk);
-        }
+        if (valid && r.k > 0)
+            collapse_write(p, r, i, n_in, base, tile_prefix + local_excl, items_out);
         if (valid && i == n_in - 1) {
-            p.level_count[level + 1] = tile_prefix + local_excl + k_int;
+            p.level_count[level + 1] = tile_prefix + local_excl + r.internal;
             p.level_base[level + 1] = base + n_in;
         }
+    }
+}
+
+// Levels [first, last) by one block, until one is empty: narrow levels (the top of a tree, its bottom, all
+// of a small one) are a chain of dependent steps, and a launch per level adds its own latency to each. A
+// barrier takes the place of the launch and a running sum that of the look-back.
+constexpr int k_narrow_block = 1024;
+// Trees of at most this many triangles are narrow throughout: 5,120 triangles, 32 launches 190 us of
+// (serialised) device time, one launch 60 us; the launches win from some 20,000 triangles on.
+constexpr std::uint64_t k_narrow_leaves = 16384;
+// Levels of at most 4^level nodes that the top block takes (level 4 has up to 256).
+constexpr int k_narrow_top = 5;
+
+__global__ void __launch_bounds__(k_narrow_block) k_collapse_narrow(collapse_params p, int first, int last) {
+    __shared__ std::uint32_t s_scan[k_narrow_block / 32];
+    unsigned const tid = threadIdx.x;
+    for (int level = first; level < last; ++level) {
+        std::uint32_t const n_in = collapse_level_items(p, level);
+        if (n_in == 0u)
+            return;
+        std::uint32_t const base = *reinterpret_cast<volatile std::uint32_t *>(&p.level_base[level]);
+        bool const odd = (level & 1) != 0;
+        collapse_item const *items_in = odd ? p.lists[1] : p.lists[0];
+        collapse_item *items_out = odd ? p.lists[0] : p.lists[1];
+        std::uint32_t done = 0; // internal children of the tiles before
+        for (std::uint32_t t = 0; t < n_in; t += k_narrow_block) {
+            std::uint32_t const i = t + tid;
+            bool const valid = i < n_in;
+            collapse_choice const r = collapse_choose(p, items_in, i, valid);
+            std::uint32_t total;
+            std::uint32_t const excl = collapse_scan<k_narrow_block>(r.internal, s_scan, total);
+            if (valid && r.k > 0)
+                collapse_write(p, r, i, n_in, base, done + excl, items_out);
+            done += total;
+            __syncthreads();
+        }
+        if (tid == 0) {
+            p.level_count[level + 1] = done;
+            p.level_base[level + 1] = base + n_in;
+        }
+        __syncthreads();
     }
 }
 
@@ -684,9 +754,24 @@ int collapse_to_bvh4(binary_node const *binary, aabb const *binary_bounds, aabb 
         std::min<std::uint64_t>(max_tiles, static_cast<std::uint64_t>(device_sm_count()) * 4));
     int level = 0;
     for (;;) {
-        int const batch = sync && level > 0 ? 8 : k_async_levels;
-        for (int b = 0; b < batch && level < k_max_levels; ++b, ++level)
-            note_launch(), k_collapse_level<<<grid, k_block, 0, s>>>(p, level);
+        if (level == 0) {
+            // the top (or all of a small tree) by one block, the levels up to log2 of the leaf count --
+            // deeper than collapsed trees commonly are -- by a launch each, the rest by one block again
+            int wide_end = k_narrow_top;
+            if (leaf_count > k_narrow_leaves)
+                while (wide_end < k_async_levels && (std::uint64_t(1) << wide_end) < leaf_count)
+                    ++wide_end;
+            int const top = leaf_count > k_narrow_leaves ? k_narrow_top : k_async_levels;
+            note_launch(), k_collapse_narrow<<<1, k_narrow_block, 0, s>>>(p, 0, top);
+            for (level = top; level < wide_end; ++level)
+                note_launch(), k_collapse_level<<<grid, k_block, 0, s>>>(p, level);
+            if (level < k_async_levels)
+                note_launch(), k_collapse_narrow<<<1, k_narrow_block, 0, s>>>(p, level, k_async_levels);
+            level = k_async_levels;
+        } else {
+            for (int b = 0; b < 8 && level < k_max_levels; ++b, ++level)
+                note_launch(), k_collapse_level<<<grid, k_block, 0, s>>>(p, level);
+        }
         GWNB_CUDA_TRY(cudaGetLastError());
         if (!sync)
             break;
