@@ -1299,20 +1299,22 @@ template <int Order, int Cap, int Mode>
 int launch_batch_cap(batch_query_state const &st, batch_query_config const &c, cudaStream_t s) {
     auto const *meshes = static_cast<taylor_params const *>(c.sorted ? st.meshes : st.meshes_unsorted);
     int const block = c.block;
+    // stack columns of the per-thread walk: the batch's largest stack bound (every mesh's thread_stack_cap)
+    int const column = st.max_stack_bound > 0 && st.max_stack_bound < Cap ? st.max_stack_bound : Cap;
+    std::size_t const smem = c.per_thread == 0 ? 0 : static_cast<std::size_t>(column) * block * sizeof(std::uint32_t);
+    auto kern = c.per_thread == 0 ? k_batch_taylor_warp<Order, Cap, Mode> : k_batch_taylor_thread<Order, Cap, Mode>;
+    if (smem > 48 * 1024)
+        GWNB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    // The blocks stride over equal shares of the warps, so a grid that is not a multiple of what is
+    // resident ends in a wave of as much work per block on part of the GPU: 8 blocks per SM where 5 are
+    // resident take two waves for 1.6. The asked number is rounded up to whole waves.
+    int resident = 0;
+    GWNB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, block, smem));
+    int const waves = (std::max(c.grid_scale, 1) + std::max(resident, 1) - 1) / std::max(resident, 1);
     std::uint64_t const need = (st.warps * 32 + block - 1) / block;
-    std::uint64_t const cap = static_cast<std::uint64_t>(device_sm_count()) * std::max(c.grid_scale, 1);
+    std::uint64_t const cap = static_cast<std::uint64_t>(device_sm_count()) * waves * std::max(resident, 1);
     unsigned const grid = static_cast<unsigned>(std::max<std::uint64_t>(std::min(need, cap), 1));
-    if (c.per_thread == 0) {
-        note_launch(), k_batch_taylor_warp<Order, Cap, Mode><<<grid, block, 0, s>>>(meshes, st.warp_begin, st.mesh_count, st.warps);
-    } else {
-        // stack columns of the batch's largest stack bound (every mesh's thread_stack_cap)
-        int const column = st.max_stack_bound > 0 && st.max_stack_bound < Cap ? st.max_stack_bound : Cap;
-        std::size_t const smem = static_cast<std::size_t>(column) * block * sizeof(std::uint32_t);
-        auto kern = k_batch_taylor_thread<Order, Cap, Mode>;
-        if (smem > 48 * 1024)
-            GWNB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-        note_launch(), kern<<<grid, block, smem, s>>>(meshes, st.warp_begin, st.mesh_count, st.warps);
-    }
+    note_launch(), kern<<<grid, block, smem, s>>>(meshes, st.warp_begin, st.mesh_count, st.warps);
     GWNB_CUDA_TRY(cudaGetLastError());
     return GWNB_OK;
 }
