@@ -533,139 +533,159 @@ struct moment_params {
     unsigned int *status;
 };
 
-template <int Order> __device__ inline void store_payload_cg(payload<Order> *dst, payload<Order> const &v) {
+// A node's payload in memory: its floats padded to whole 128-bit words.
+template <int Order> constexpr int k_payload_words = (static_cast<int>(sizeof(payload<Order>)) + 15) / 16;
+
+template <int Order> __device__ inline void store_payload_cg(float4 *dst, payload<Order> const &v) {
+    constexpr int n = static_cast<int>(sizeof(payload<Order>) / 4);
     float const *s = reinterpret_cast<float const *>(&v);
-    float *d = reinterpret_cast<float *>(dst);
 #pragma unroll
-    for (int k = 0; k < static_cast<int>(sizeof(payload<Order>) / 4); ++k)
-        __stcg(d + k, s[k]);
+    for (int k = 0; k < k_payload_words<Order>; ++k)
+        __stcg(dst + k, make_float4(s[4 * k], 4 * k + 1 < n ? s[4 * k + 1] : 0.0f, 4 * k + 2 < n ? s[4 * k + 2] : 0.0f,
+                                    4 * k + 3 < n ? s[4 * k + 3] : 0.0f));
 }
-template <int Order> __device__ inline payload<Order> load_payload_cg(payload<Order> const *src) {
+template <int Order> __device__ inline payload<Order> load_payload_cg(float4 const *src) {
+    constexpr int n = static_cast<int>(sizeof(payload<Order>) / 4);
     payload<Order> v;
-    float const *s = reinterpret_cast<float const *>(src);
     float *d = reinterpret_cast<float *>(&v);
 #pragma unroll
-    for (int k = 0; k < static_cast<int>(sizeof(payload<Order>) / 4); ++k)
-        d[k] = __ldcg(s + k);
+    for (int k = 0; k < k_payload_words<Order>; ++k) {
+        float4 const w = __ldcg(src + k);
+        d[4 * k] = w.x;
+        if (4 * k + 1 < n)
+            d[4 * k + 1] = w.y;
+        if (4 * k + 2 < n)
+            d[4 * k + 2] = w.z;
+        if (4 * k + 3 < n)
+            d[4 * k + 3] = w.w;
+    }
     return v;
 }
 
-// s_even is this thread's column of a [k_qnode_components][blockDim.x] shared-memory array: the even
-// slot's sidecar components wait there for the odd slot's, so that a pair is stored in 128-bit words.
+// Finishes node n by the four lanes of `quad`, lane s of them its child slot s: the slot's payload (from
+// its triangles or the child node's), its coefficients in both layouts, and the node's total, summed
+// over the lanes ((0 + 1) + (2 + 3); an empty slot adds 0). A field's four slots lie side by side in the
+// published layout; for the sidecar the lanes of a pair exchange halves, so that each stores whole
+// 128-bit words.
 template <int Order>
-__device__ inline void finish_node(moment_params const &p, std::uint32_t n, float *s_even) {
+__device__ inline void finish_node(moment_params const &p, std::uint32_t n, int s, unsigned quad) {
     constexpr int F = Order == 0 ? 7 : (Order == 1 ? 13 : 23);
     constexpr int Q = qnode_traits<Order>::k_f4_per_child;
-    payload<Order> *pend = static_cast<payload<Order> *>(p.pending);
-    payload<Order> total{};
-    bool init = false;
-    float *ref = p.ref_nodes + static_cast<std::uint64_t>(n) * F * 4;
-    float4 *qn = p.qnodes + static_cast<std::uint64_t>(n) * 4 * Q;
-#pragma unroll 1
-    for (int s = 0; s < 4; ++s) {
-        node4 const &nd = p.nodes[n];
-        std::uint64_t const r = nd.c[s].reference;
-        float q[Q * 4];
+    float4 *pend = static_cast<float4 *>(p.pending);
+    std::uint64_t const r = p.nodes[n].c[s].reference;
+    payload<Order> m{};
+    coeffs<Order> c{};
+    float q[Q * 4];
 #pragma unroll
-        for (int k = 0; k < Q * 4; ++k)
-            q[k] = 0.0f;
-        if (!ref_valid(r)) {
-#pragma unroll
-            for (int f = 0; f < F; ++f)
-                ref[f * 4 + s] = 0.0f;
-            q[3] = -1.0f;
-            q[7] = __uint_as_float(k_invalid_u32);
-            p.qcounts[n * 4 + s] = 0u;
-        } else {
-            payload<Order> m{};
-            std::uint32_t qref = 0;
-            if (ref_internal(r)) {
-                std::uint64_t const c = ref_offset(r);
-                if (c < p.node_count)
-                    m = load_payload_cg(pend + c);
-                else
-                    atomicOr(p.status, k_err_topology);
-                qref = static_cast<std::uint32_t>(c) & k_qref_index_mask;
-                p.qcounts[n * 4 + s] = 0u;
-            } else {
-                std::uint64_t const first = ref_offset(r);
-                std::uint32_t const cnt = ref_count(r);
-                for (std::uint32_t k = 0; k < cnt; ++k) {
-                    std::uint64_t const si = first + k;
-                    if (si >= p.primitive_count) {
-                        atomicOr(p.status, k_err_topology);
-                        break;
-                    }
-                    payload<Order> const tm = triangle_moment<Order>(p.triangles[si]);
-                    if (k == 0)
-                        m = tm;
-                    else
-                        accumulate(m, tm);
-                }
-                qref = k_qref_leaf | (static_cast<std::uint32_t>(first) & k_qref_index_mask) |
-                       (cnt > 1 ? k_qref_multi : 0u);
-                p.qcounts[n * 4 + s] = cnt;
-            }
-            aabb const b = load_bounds_cg(p.nodes, n, s);
-            coeffs<Order> const c = finalize_slot<Order>(b, m);
-#pragma unroll
-            for (int f = 0; f < F; ++f)
-                ref[f * 4 + s] = c.f[f];
-            q[0] = -c.f[1];
-            q[1] = -c.f[2];
-            q[2] = -c.f[3];
-            q[3] = c.f[0];
-            q[4] = -c.f[4];
-            q[5] = -c.f[5];
-            q[6] = -c.f[6];
-            q[7] = __uint_as_float(qref);
-            if constexpr (Order >= 1)
-                fold_far_field_coefficients<Order>(c, q + 8);
-            if (init)
-                accumulate(total, m);
+    for (int k = 0; k < Q * 4; ++k)
+        q[k] = 0.0f;
+    q[3] = -1.0f;
+    q[7] = __uint_as_float(k_invalid_u32);
+    std::uint32_t cnt = 0;
+    if (ref_valid(r)) {
+        std::uint32_t qref = 0;
+        if (ref_internal(r)) {
+            std::uint64_t const child = ref_offset(r);
+            if (child < p.node_count)
+                m = load_payload_cg<Order>(pend + child * k_payload_words<Order>);
             else
-                total = m;
-            init = true;
-        }
-        if ((s & 1) == 0) {
-#pragma unroll
-            for (int k = 0; k < Q * 4; ++k)
-                s_even[k * blockDim.x] = q[k];
+                atomicOr(p.status, k_err_topology);
+            qref = static_cast<std::uint32_t>(child) & k_qref_index_mask;
         } else {
-#pragma unroll
-            for (int k = 0; k < Q * 2; ++k)
-                qn[(s >> 1) * 2 * Q + k] = make_float4(s_even[2 * k * blockDim.x], q[2 * k],
-                                                       s_even[(2 * k + 1) * blockDim.x], q[2 * k + 1]);
+            std::uint64_t const first = ref_offset(r);
+            cnt = ref_count(r);
+            for (std::uint32_t k = 0; k < cnt; ++k) {
+                std::uint64_t const si = first + k;
+                if (si >= p.primitive_count) {
+                    atomicOr(p.status, k_err_topology);
+                    break;
+                }
+                payload<Order> const tm = triangle_moment<Order>(p.triangles[si]);
+                if (k == 0)
+                    m = tm;
+                else
+                    accumulate(m, tm);
+            }
+            qref = k_qref_leaf | (static_cast<std::uint32_t>(first) & k_qref_index_mask) | (cnt > 1 ? k_qref_multi : 0u);
         }
+        c = finalize_slot<Order>(load_bounds_cg(p.nodes, n, s), m);
+        q[0] = -c.f[1];
+        q[1] = -c.f[2];
+        q[2] = -c.f[3];
+        q[3] = c.f[0];
+        q[4] = -c.f[4];
+        q[5] = -c.f[5];
+        q[6] = -c.f[6];
+        q[7] = __uint_as_float(qref);
+        if constexpr (Order >= 1)
+            fold_far_field_coefficients<Order>(c, q + 8);
     }
-    store_payload_cg(pend + n, total);
+    p.qcounts[n * 4 + s] = cnt;
+    float *ref = p.ref_nodes + static_cast<std::uint64_t>(n) * F * 4;
+#pragma unroll
+    for (int f = 0; f < F; ++f)
+        ref[f * 4 + s] = c.f[f];
+    // word k of a pair holds components 2k and 2k + 1 of its even and its odd slot: the even lane stores
+    // the first half of the words, the odd lane the second
+    bool const odd = (s & 1) != 0;
+    float4 *const qn = p.qnodes + static_cast<std::uint64_t>(n) * 4 * Q + (s >> 1) * 2 * Q + (odd ? Q : 0);
+#pragma unroll
+    for (int k = 0; k < Q; ++k) {
+        float const x = __shfl_xor_sync(quad, odd ? q[2 * k] : q[2 * Q + 2 * k], 1);
+        float const y = __shfl_xor_sync(quad, odd ? q[2 * k + 1] : q[2 * Q + 2 * k + 1], 1);
+        float const u = odd ? q[2 * Q + 2 * k] : q[2 * k], v = odd ? q[2 * Q + 2 * k + 1] : q[2 * k + 1];
+        qn[k] = odd ? make_float4(x, u, y, v) : make_float4(u, x, v, y);
+    }
+    float *t = reinterpret_cast<float *>(&m);
+#pragma unroll
+    for (int k = 0; k < static_cast<int>(sizeof(payload<Order>) / 4); ++k) {
+        t[k] += __shfl_xor_sync(quad, t[k], 1);
+        t[k] += __shfl_xor_sync(quad, t[k], 2);
+    }
+    if (s == 0)
+        store_payload_cg<Order>(pend + static_cast<std::uint64_t>(n) * k_payload_words<Order>, m);
 }
 
-// One work item of the moment refit: from leaf-bearing node t, finish every node this thread is
-// the last arrival at, climbing to the root.
-template <int Order>
-__device__ __forceinline__ void refit_moments_item(moment_params const &p, std::uint64_t t, float *s_even) {
+// One work item of the moment refit, by four lanes: from leaf-bearing node t, finish every node these
+// are the last to arrive at, climbing to the root. A climb is a chain of dependent loads and arrivals, so
+// its time is the latency of a step: one lane per slot takes a quarter of the arithmetic and of the
+// loads of one thread per node, and its stores are contiguous. 1M triangles, orders 0 / 1 / 2: 0.26 /
+// 0.41 / 0.70 ms with one thread per node, 0.19 / 0.26 / 0.49 ms so; 5,120 triangles: 53 / 60 / 90 us and
+// 33 / 35 / 42 us.
+template <int Order> __device__ __forceinline__ void refit_moments_item(moment_params const &p, std::uint64_t t) {
+    unsigned const lane = threadIdx.x & 31u;
+    int const s = static_cast<int>(lane & 3u);
+    unsigned const quad = 0xfu << (lane & ~3u);
     std::uint32_t cur = p.leaf_nodes[t];
     std::uint64_t guard = 0;
     for (;;) {
+        // each lane's stores are released by its own fence and ordered before the arrival by the warp
+        // barrier; after it the same the other way round
         fence_acq_rel_gpu();
-        std::uint32_t const arrived = atomicAdd(&p.arrivals[cur], 1u) + 1u;
+        __syncwarp(quad);
+        std::uint32_t arrived = 0;
+        if (s == 0)
+            arrived = atomicAdd(&p.arrivals[cur], 1u) + 1u;
+        arrived = __shfl_sync(quad, arrived, static_cast<int>(lane & ~3u));
         std::uint32_t const expect = p.expected[cur];
         if (arrived < expect)
             return;
         if (arrived > expect) {
-            atomicOr(p.status, k_err_topology);
+            if (s == 0)
+                atomicOr(p.status, k_err_topology);
             return;
         }
-        p.arrivals[cur] = 0u;
+        if (s == 0)
+            p.arrivals[cur] = 0u;
         fence_acq_rel_gpu();
-        finish_node<Order>(p, cur, s_even);
+        finish_node<Order>(p, cur, s, quad);
         std::uint32_t const ps = p.parent_slot[cur];
         if (ps == k_invalid_u32)
             return;
         std::uint32_t const parent = ps >> 2;
         if (parent >= p.node_count || ++guard > p.node_count) {
-            atomicOr(p.status, k_err_topology);
+            if (s == 0)
+                atomicOr(p.status, k_err_topology);
             return;
         }
         cur = parent;
@@ -673,10 +693,9 @@ __device__ __forceinline__ void refit_moments_item(moment_params const &p, std::
 }
 
 template <int Order> __global__ void __launch_bounds__(k_block) k_refit_moments(moment_params p) {
-    __shared__ float s_even[k_qnode_components<Order> * k_block];
-    std::uint64_t const t = static_cast<std::uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    std::uint64_t const t = (static_cast<std::uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 2;
     if (t < p.leaf_node_count)
-        refit_moments_item<Order>(p, t, s_even + threadIdx.x);
+        refit_moments_item<Order>(p, t);
 }
 
 // ---- batched refit (many BVHs, one launch) -------------------------------------------------------
@@ -726,12 +745,11 @@ template <int Order>
 __global__ void __launch_bounds__(k_batch_block_max)
     k_batch_refit_moments(moment_params const *__restrict__ meshes, std::uint64_t const *__restrict__ begin,
                           std::uint32_t mesh_count) {
-    __shared__ float s_even[k_qnode_components<Order> * k_batch_block_max];
-    std::uint64_t const total = begin[mesh_count];
-    for (std::uint64_t i = static_cast<std::uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-         i += static_cast<std::uint64_t>(gridDim.x) * blockDim.x) {
+    std::uint64_t const total = begin[mesh_count]; // items of four lanes each
+    for (std::uint64_t i = (static_cast<std::uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 2; i < total;
+         i += (static_cast<std::uint64_t>(gridDim.x) * blockDim.x) >> 2) {
         std::uint32_t const m = find_mesh(begin, mesh_count, i);
-        refit_moments_item<Order>(meshes[m], i - begin[m], s_even + threadIdx.x);
+        refit_moments_item<Order>(meshes[m], i - begin[m]);
     }
 }
 
@@ -948,7 +966,7 @@ int batch_refit_launch(batch_refit_state const &st, int block, bool bounds, bool
             static_cast<batch_bounds_mesh const *>(st.bounds_meshes), st.bounds_begin, st.mesh_count);
     if (moments && st.moment_items > 0) {
         auto const *md = static_cast<moment_params const *>(st.moment_meshes);
-        unsigned const g = grid(st.moment_items);
+        unsigned const g = grid(4 * st.moment_items);
         switch (st.order) {
         case 0: note_launch(), k_batch_refit_moments<0><<<g, block, 0, s>>>(md, st.moment_begin, st.mesh_count); break;
         case 1: note_launch(), k_batch_refit_moments<1><<<g, block, 0, s>>>(md, st.moment_begin, st.mesh_count); break;
@@ -1016,7 +1034,7 @@ int refit_moments_async(gwnb_bvh4_f32 const *bvh, gwnb_moment4_f32 *m, cudaStrea
     p.qcounts = ma->qcounts;
     p.pending = ma->payload;
     p.status = a->status;
-    unsigned const grid = grid_for(a->leaf_node_count);
+    unsigned const grid = grid_for(4 * a->leaf_node_count); // four lanes per item
     if (grid == 0)
         return set_error(GWNB_INTERNAL_ERROR, "bvh.refit.moment: BVH has no leaf-bearing node.");
     switch (m->order) {
@@ -1029,7 +1047,7 @@ int refit_moments_async(gwnb_bvh4_f32 const *bvh, gwnb_moment4_f32 *m, cudaStrea
 }
 
 std::size_t moment_payload_bytes(int order) {
-    return order == 0 ? sizeof(payload<0>) : (order == 1 ? sizeof(payload<1>) : sizeof(payload<2>));
+    return 16u * (order == 0 ? k_payload_words<0> : (order == 1 ? k_payload_words<1> : k_payload_words<2>));
 }
 
 } // namespace gwnb
