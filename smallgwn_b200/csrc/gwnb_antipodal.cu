@@ -495,9 +495,9 @@ __device__ __forceinline__ row_pair load_row_pair(float const *p) {
 // Singular on +z (classify): a collinear projection whose ends lie on opposite sides of the query.
 __device__ __forceinline__ bool row_singular(float det, float c0) { return det == 0.0f && c0 <= 0.0f; }
 
-// A pair's angles: residuals times multiplicity added to sum, quarters times multiplicity to quarters.
-// True when a half is singular or opposed: nothing is added and the caller takes the rows one by one.
-__device__ __forceinline__ bool area_pair(row_pair const &t, x2::f2 nqx, x2::f2 nqy, x2::f2 nqz, double &sum,
+// A pair's angles: residuals times multiplicity r, quarters times multiplicity k. True when a half is
+// singular or opposed: r and k then mean nothing and the caller takes the rows one by one.
+__device__ __forceinline__ bool area_pair(row_pair const &t, x2::f2 nqx, x2::f2 nqy, x2::f2 nqz, float &r0, float &r1,
                                           float &quarters) {
     using namespace x2;
     f2 const sx = add(t.sx, nqx), sy = add(t.sy, nqy), sz = add(t.sz, nqz);
@@ -511,8 +511,7 @@ __device__ __forceinline__ bool area_pair(row_pair const &t, x2::f2 nqx, x2::f2 
     float d0, d1, o0, o1;
     unpack(det, d0, d1);
     unpack(fma(fma(sz, ez, c0), rr, both(1.0f)), o0, o1);
-    if (fminf(fabsf(d0), fabsf(d1)) == 0.0f || fminf(o0, o1) < k_ap_opposed)
-        return true;
+    bool const apart = fminf(fabsf(d0), fabsf(d1)) == 0.0f || fminf(o0, o1) < k_ap_opposed;
     f2 const us = mul(mul(ps, rs), rs), ue = mul(mul(pe, re), re);
     float z0, z1, u0, u1, gs0, gs1, hs0, hs1, ge0, ge1, he0, he1;
     unpack(mul(sz, rs), z0, z1);
@@ -526,7 +525,7 @@ __device__ __forceinline__ bool area_pair(row_pair const &t, x2::f2 nqx, x2::f2 
     f2 const kk = mul(rr, mul(pack(gs0, gs1), pack(ge0, ge1)));
     f2 const num = mul(det, mul(kk, both(-1.0f)));
     f2 const den = fma(c0, kk, mul(pack(hs0, hs1), pack(he0, he1)));
-    float n0, n1, e0, e1, r0, r1, k0, k1, m0, m1;
+    float n0, n1, e0, e1, k0, k1, m0, m1;
     unpack(num, n0, n1);
     unpack(den, e0, e1);
     f2 const lo = pack(fminf(fabsf(n0), fabsf(e0)), fminf(fabsf(n1), fabsf(e1)));
@@ -535,10 +534,8 @@ __device__ __forceinline__ bool area_pair(row_pair const &t, x2::f2 nqx, x2::f2 
     unpack(t.m, m0, m1);
     quadrant(n0, e0, r0, k0);
     quadrant(n1, e1, r1, k1);
-    sum += static_cast<double>(r0);
-    sum += static_cast<double>(r1);
-    quarters = __fmaf_rn(k1, m1, __fmaf_rn(k0, m0, quarters));
-    return false;
+    quarters = __fmaf_rn(k1, m1, __fmul_rn(k0, m0));
+    return apart;
 }
 
 // Value batch (:533-568), one query per thread: crossings per thread, then the boundary rows in tiles
@@ -567,20 +564,36 @@ __global__ void __launch_bounds__(256) k_antipodal(antipodal_params p) {
             s_dyn[t] = __ldg(reinterpret_cast<float4 const *>(p.edges + base / 2 * k_row_pair) + t);
         __syncthreads();
         float quarters = 0.0f;
-        for (int j = 0; j < pairs; ++j) {
-            if (!area_pair(load_row_pair(s_rows + j * k_row_pair), nqx, nqy, nqz, sum, quarters))
-                continue;
-            for (int h = 0; h < 2 && rc == 0; ++h) {
-                std::uint64_t const i = base + static_cast<std::uint64_t>(2 * j + h);
-                if (i >= p.edge_count)
+        // two pairs at a time, so that their chains interleave
+        for (int j = 0; j < pairs; j += 2) {
+            float r[2][2], k[2];
+            bool apart[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) // an odd last pair is taken twice, the second time for nothing
+                apart[u] = area_pair(load_row_pair(s_rows + (j + u < pairs ? j + u : j) * k_row_pair), nqx, nqy, nqz,
+                                     r[u][0], r[u][1], k[u]);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                if (j + u >= pairs)
                     break;
-                float4 A, B;
-                load_row(p.edges, i, A, B);
-                double term;
-                if (row_term<2>(A, B, q, term))
-                    sum += 0.5 * term;
-                else
-                    rc = 1;
+                if (!apart[u]) {
+                    sum += static_cast<double>(r[u][0]);
+                    sum += static_cast<double>(r[u][1]);
+                    quarters += k[u];
+                    continue;
+                }
+                for (int h = 0; h < 2 && rc == 0; ++h) {
+                    std::uint64_t const i = base + static_cast<std::uint64_t>(2 * (j + u) + h);
+                    if (i >= p.edge_count)
+                        break;
+                    float4 A, B;
+                    load_row(p.edges, i, A, B);
+                    double term;
+                    if (row_term<2>(A, B, q, term))
+                        sum += 0.5 * term;
+                    else
+                        rc = 1;
+                }
             }
         }
         turns += static_cast<double>(quarters);
@@ -736,8 +749,8 @@ __device__ __forceinline__ void edge_gradient_d(float4 A, float4 B, v3 q, double
         g[k] = f * c[k];
 }
 
-// True when a half is singular or opposed (see area_pair).
-__device__ __forceinline__ bool gradient_pair(grad_pair const &t, x2::f2 nqx, x2::f2 nqy, x2::f2 nqz, double (&g)[3]) {
+// A pair's gradients c. True when a half is singular or opposed (see area_pair).
+__device__ __forceinline__ bool gradient_pair(grad_pair const &t, x2::f2 nqx, x2::f2 nqy, x2::f2 nqz, x2::f2 (&c)[3]) {
     using namespace x2;
     f2 const sx = add(t.r.sx, nqx), sy = add(t.r.sy, nqy), sz = add(t.r.sz, nqz);
     f2 const ex = add(t.r.ex, nqx), ey = add(t.r.ey, nqy), ez = add(t.r.ez, nqz);
@@ -748,19 +761,11 @@ __device__ __forceinline__ bool gradient_pair(grad_pair const &t, x2::f2 nqx, x2
     unpack(det, d0, d1);
     f2 const o = fma(dot(sx, sy, sz, ex, ey, ez), rr, both(1.0f));
     unpack(o, o0, o1);
-    if (fminf(fabsf(d0), fabsf(d1)) == 0.0f || fminf(o0, o1) < k_grad_opposed)
-        return true;
     f2 const f = divide(mul(mul(add(rs, re), rr), t.r.m), o);
-    f2 const c[3] = {mul(fma(sy, t.lz, mul(sz, t.my)), f), mul(fma(sz, t.lx, mul(sx, t.mz)), f),
-                     mul(fma(sx, t.ly, mul(sy, t.mx)), f)};
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        float a, b;
-        unpack(c[k], a, b);
-        g[k] += static_cast<double>(a);
-        g[k] += static_cast<double>(b);
-    }
-    return false;
+    c[0] = mul(fma(sy, t.lz, mul(sz, t.my)), f);
+    c[1] = mul(fma(sz, t.lx, mul(sx, t.mz)), f);
+    c[2] = mul(fma(sx, t.ly, mul(sy, t.mx)), f);
+    return fminf(fabsf(d0), fabsf(d1)) == 0.0f || fminf(o0, o1) < k_grad_opposed;
 }
 
 __global__ void __launch_bounds__(256) k_antipodal_gradient(antipodal_params p) {
@@ -790,25 +795,44 @@ __global__ void __launch_bounds__(256) k_antipodal_gradient(antipodal_params p) 
             }
         }
         __syncthreads();
-        for (int j = 0; j < pairs; ++j) {
-            if (!gradient_pair(load_grad_pair(s_rows + j * k_grad_pair), nqx, nqy, nqz, sum))
-                continue;
-            for (int h = 0; h < 2 && ok; ++h) {
-                std::uint64_t const i = base + static_cast<std::uint64_t>(2 * j + h);
-                if (i >= p.edge_count)
-                    break;
-                float4 A, B;
-                load_row(p.edges, i, A, B);
-                v3 s, e;
-                row_ends(A, B, q, s, e);
-                if (classify<2>(s, e).singular) {
-                    ok = false;
-                } else {
-                    double g[3];
-                    edge_gradient_d(A, B, q, g);
+        for (int j = 0; j < pairs; j += 2) { // two pairs at a time, as in the value batch
+            x2::f2 c[2][3];
+            bool apart[2];
 #pragma unroll
-                    for (int k = 0; k < 3; ++k)
-                        sum[k] += g[k];
+            for (int u = 0; u < 2; ++u)
+                apart[u] = gradient_pair(load_grad_pair(s_rows + (j + u < pairs ? j + u : j) * k_grad_pair), nqx, nqy,
+                                         nqz, c[u]);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                if (j + u >= pairs)
+                    break;
+                if (!apart[u]) {
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) {
+                        float a, b;
+                        x2::unpack(c[u][k], a, b);
+                        sum[k] += static_cast<double>(a);
+                        sum[k] += static_cast<double>(b);
+                    }
+                    continue;
+                }
+                for (int h = 0; h < 2 && ok; ++h) {
+                    std::uint64_t const i = base + static_cast<std::uint64_t>(2 * (j + u) + h);
+                    if (i >= p.edge_count)
+                        break;
+                    float4 A, B;
+                    load_row(p.edges, i, A, B);
+                    v3 s, e;
+                    row_ends(A, B, q, s, e);
+                    if (classify<2>(s, e).singular) {
+                        ok = false;
+                    } else {
+                        double g[3];
+                        edge_gradient_d(A, B, q, g);
+#pragma unroll
+                        for (int k = 0; k < 3; ++k)
+                            sum[k] += g[k];
+                    }
                 }
             }
         }
