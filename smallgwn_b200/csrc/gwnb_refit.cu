@@ -536,14 +536,6 @@ struct moment_params {
 // A node's payload in memory: its floats padded to whole 128-bit words.
 template <int Order> constexpr int k_payload_words = (static_cast<int>(sizeof(payload<Order>)) + 15) / 16;
 
-template <int Order> __device__ inline void store_payload_cg(float4 *dst, payload<Order> const &v) {
-    constexpr int n = static_cast<int>(sizeof(payload<Order>) / 4);
-    float const *s = reinterpret_cast<float const *>(&v);
-#pragma unroll
-    for (int k = 0; k < k_payload_words<Order>; ++k)
-        __stcg(dst + k, make_float4(s[4 * k], 4 * k + 1 < n ? s[4 * k + 1] : 0.0f, 4 * k + 2 < n ? s[4 * k + 2] : 0.0f,
-                                    4 * k + 3 < n ? s[4 * k + 3] : 0.0f));
-}
 template <int Order> __device__ inline payload<Order> load_payload_cg(float4 const *src) {
     constexpr int n = static_cast<int>(sizeof(payload<Order>) / 4);
     payload<Order> v;
@@ -563,10 +555,9 @@ template <int Order> __device__ inline payload<Order> load_payload_cg(float4 con
 }
 
 // Finishes node n by the four lanes of `quad`, lane s of them its child slot s: the slot's payload (from
-// its triangles or the child node's), its coefficients in both layouts, and the node's total, summed
-// over the lanes ((0 + 1) + (2 + 3); an empty slot adds 0). A field's four slots lie side by side in the
-// published layout; for the sidecar the lanes of a pair exchange halves, so that each stores whole
-// 128-bit words.
+// its triangles or the child node's), its coefficients in both layouts, and the node's total. A field's
+// four slots lie side by side in the published layout; for the sidecar the lanes of a pair exchange
+// halves, so that each stores whole 128-bit words.
 template <int Order>
 __device__ inline void finish_node(moment_params const &p, std::uint32_t n, int s, unsigned quad) {
     constexpr int F = Order == 0 ? 7 : (Order == 1 ? 13 : 23);
@@ -636,14 +627,35 @@ __device__ inline void finish_node(moment_params const &p, std::uint32_t n, int 
         float const u = odd ? q[2 * Q + 2 * k] : q[2 * k], v = odd ? q[2 * Q + 2 * k + 1] : q[2 * k + 1];
         qn[k] = odd ? make_float4(x, u, y, v) : make_float4(u, x, v, y);
     }
-    float *t = reinterpret_cast<float *>(&m);
+    // The total of the node: each group of four floats is transposed across the lanes, so that lane s
+    // holds float s of all four slots, and added in slot order from the first slot that holds a child
+    // (the order in which saved scenes were summed: their moments are compared bit for bit on loading).
+    constexpr int n_floats = static_cast<int>(sizeof(payload<Order>) / 4);
+    float const *v = reinterpret_cast<float const *>(&m);
+    unsigned const held = __ballot_sync(quad, ref_valid(r)) >> (__ffs(static_cast<int>(quad)) - 1);
+    bool const high = (s & 2) != 0;
+    float *const total = reinterpret_cast<float *>(pend + static_cast<std::uint64_t>(n) * k_payload_words<Order>);
 #pragma unroll
-    for (int k = 0; k < static_cast<int>(sizeof(payload<Order>) / 4); ++k) {
-        t[k] += __shfl_xor_sync(quad, t[k], 1);
-        t[k] += __shfl_xor_sync(quad, t[k], 2);
+    for (int k = 0; k < k_payload_words<Order>; ++k) {
+        float const v0 = v[4 * k], v1 = 4 * k + 1 < n_floats ? v[4 * k + 1] : 0.0f,
+                    v2 = 4 * k + 2 < n_floats ? v[4 * k + 2] : 0.0f, v3 = 4 * k + 3 < n_floats ? v[4 * k + 3] : 0.0f;
+        // with the pair's other lane: floats 0 and 2 to the even lane, 1 and 3 to the odd one
+        float const x = __shfl_xor_sync(quad, odd ? v0 : v1, 1), y = __shfl_xor_sync(quad, odd ? v2 : v3, 1);
+        float const a0 = odd ? x : v0, a1 = odd ? v1 : x; // float (s & 1) of the pair's even and odd slot
+        float const b0 = odd ? y : v2, b1 = odd ? v3 : y; // float 2 + (s & 1)
+        // with the other pair: the lower floats to the lower pair
+        float const p0 = __shfl_xor_sync(quad, high ? a0 : b0, 2), p1 = __shfl_xor_sync(quad, high ? a1 : b1, 2);
+        float const w[4] = {high ? p0 : a0, high ? p1 : a1, high ? b0 : p0, high ? b1 : p1};
+        float t = 0.0f;
+        bool any = false;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            bool const in = ((held >> c) & 1u) != 0u;
+            t = in ? (any ? t + w[c] : w[c]) : t;
+            any = any || in;
+        }
+        __stcg(total + 4 * k + s, t);
     }
-    if (s == 0)
-        store_payload_cg<Order>(pend + static_cast<std::uint64_t>(n) * k_payload_words<Order>, m);
 }
 
 // One work item of the moment refit, by four lanes: from leaf-bearing node t, finish every node these
@@ -692,7 +704,8 @@ template <int Order> __device__ __forceinline__ void refit_moments_item(moment_p
     }
 }
 
-template <int Order> __global__ void __launch_bounds__(k_block) k_refit_moments(moment_params p) {
+// Four blocks per SM: at most 128 registers (order 2 takes 132 by itself, three blocks and a quarter more time).
+template <int Order> __global__ void __launch_bounds__(k_block, 4) k_refit_moments(moment_params p) {
     std::uint64_t const t = (static_cast<std::uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 2;
     if (t < p.leaf_node_count)
         refit_moments_item<Order>(p, t);
