@@ -13,8 +13,8 @@
 // The collapse itself is restructured: every tree level allocates its child node ids with a
 // decoupled look-back scan, which yields a canonical breadth-first node order directly (no
 // persistent work queue, no reorder sort). A build enqueues the first 32 levels without a host
-// round trip (a level past the bottom exits at once) and learns from its single read-back whether
-// the tree was deeper.
+// round trip (narrow ones by one block in one launch; a level past the bottom exits at once) and learns
+// from its single read-back whether the tree was deeper.
 #include "gwnb_internal.cuh"
 
 #include <algorithm>

@@ -212,11 +212,11 @@ __device__ __forceinline__ float point_triangle_d2(v3 p, v3 a, v3 b, v3 c) {
 // Nodes after which a query's own walk, and a warp's union walk, is given up to k_distance_long. A
 // query near the middle of a round mesh has most of the surface at about its distance: on the 1M-triangle
 // sphere the mean is 240 nodes, the longest query takes 9,600, and a batch of 2M ended 30 ms after the
-// work of all other warps. 2M ordered / 500k unordered / 50k ordered queries: 54.9 / 20.0 / 10.0 ms without,
-// 26.4 / 8.3 / 1.7 ms with 128 and 512 nodes, 26.8 / 10.2 / 2.7 with 256 and 1,024, 29.9 / 13.4 / 6.5 with
-// 1,024 and 4,096.
-constexpr int k_alone_nodes = 128;
-constexpr int k_union_nodes = 512;
+// work of all other warps. Two shapes of 2M ordered, 500k unordered and 50k ordered queries: 54.9, 14.4,
+// 20.0 and 10.0 ms without; 22.6, 13.7, 7.1 and 1.2 ms with 64 and 256 nodes, 24.5, 13.1, 7.5 and 1.4 with 96
+// and 384, 26.0, 12.7, 8.0 and 1.7 with 128 and 512, 29.9, 14.1, 13.4 and 6.5 with 1,024 and 4,096.
+constexpr int k_alone_nodes = 64;
+constexpr int k_union_nodes = 256;
 
 // The state of one distance query between node visits (see ray_lane).
 struct distance_lane {
@@ -915,19 +915,25 @@ template <int Cap> __global__ void __launch_bounds__(256, 4) k_distance_warp(spa
 
 // One query per warp: the queries k_distance_warp gave up, or all of a batch too small to fill the GPU
 // (long_items == nullptr). The lanes take the warp's 32 uppermost stack entries at a time (node and box
-// distance, in shared memory), test their children against the warp's common bound, evaluate the leaf
-// children and push the internal ones, nearest uppermost, so that a query of thousands of nodes takes
-// some hundred steps. A minimum does not depend on the order of the triangles, so the result is the same.
+// distance, in shared memory), test their children against the warp's common bound, collect the triangles
+// of the leaf children, tested 32 at a time, and push the internal ones, nearest uppermost, so that a query
+// of thousands of nodes takes some hundred steps. A minimum does not depend on the order of the
+// triangles, so the result is the same. (Tested slot by slot by the lanes that met them, the triangles
+// took more than half of the instructions: 14.1 ms of a 26 ms batch.)
 constexpr int k_long_block = 256;
-constexpr int k_long_stack = 512; // entries per warp
+constexpr int k_long_stack = 512;  // entries per warp
+constexpr int k_long_leaves = 160; // triangles waiting per warp: fewer than 32, and up to 128 of a step
 
 __global__ void __launch_bounds__(k_long_block) k_distance_long(spatial_params p) {
     __shared__ std::uint32_t s_node[k_long_block / 32][k_long_stack];
     __shared__ float s_key[k_long_block / 32][k_long_stack];
+    __shared__ std::uint32_t s_leaf[k_long_block / 32][k_long_leaves];
     constexpr unsigned all = 0xffffffffu;
     unsigned const lane = threadIdx.x & 31u;
     std::uint32_t *const nodes = s_node[threadIdx.x >> 5];
     float *const keys = s_key[threadIdx.x >> 5];
+    std::uint32_t *const tris = s_leaf[threadIdx.x >> 5];
+    unsigned const before = (1u << lane) - 1u;
     unsigned const total = p.long_items != nullptr ? *p.long_count : static_cast<unsigned>(p.n);
     for (;;) {
         unsigned item = 0;
@@ -961,7 +967,24 @@ __global__ void __launch_bounds__(k_long_block) k_distance_long(spatial_params p
         // above this height only one entry is taken at a time: a depth-first walk from there adds at
         // most the tree's stack bound and the last node's children
         int const high = k_long_stack - p.stack_cap - 4;
-        while (sp > 0) {
+        int leaves = 0; // triangles waiting in tris
+        // Tests the last (up to 32) of them and brings the lanes to their common bound.
+        auto test = [&]() {
+            __syncwarp();
+            int const from = leaves > 32 ? leaves - 32 : 0;
+            if (from + static_cast<int>(lane) < leaves) {
+                v3 a, b, c;
+                record_vertices(p.tri48, tris[from + static_cast<int>(lane)], a, b, c);
+                float const d2 = point_triangle_d2(L.q, a, b, c);
+                if (d2 < L.best)
+                    L.best = d2;
+            }
+            leaves = from;
+            // squared distances are not negative, so their bits order like the values
+            L.best = __uint_as_float(__reduce_min_sync(all, __float_as_uint(L.best)));
+            L.touched = !(L.best > 0.0f);
+        };
+        while (sp > 0 && !L.touched) {
             int n = sp < 32 ? sp : 32;
             if (sp + 3 * n > high)
                 n = sp < high - 3 ? (high - sp) / 3 : 1;
@@ -972,6 +995,8 @@ __global__ void __launch_bounds__(k_long_block) k_distance_long(spatial_params p
             __syncwarp();
             cand4 cd;
             int cnt = 0;
+            std::uint32_t tri[4] = {0, 0, 0, 0};
+            bool leaf[4] = {false, false, false, false};
             if (take && key < L.best && node < p.node_count) {
                 float4 const *nd = p.nodes + static_cast<std::uint64_t>(node) * 8;
 #pragma unroll
@@ -985,16 +1010,28 @@ __global__ void __launch_bounds__(k_long_block) k_distance_long(spatial_params p
                     if (!(d2 < L.best))
                         continue;
                     if (ref_leaf(ref)) {
-                        distance_leaf<false>(p, L, ref);
+                        tri[s] = static_cast<std::uint32_t>(ref_offset(ref));
+                        leaf[s] = ref_count(ref) == 1u && ref_offset(ref) < p.primitive_count;
+                        if (ref_count(ref) > 1u)
+                            distance_leaf<false>(p, L, ref);
                     } else if (ref_offset(ref) < p.node_count) {
                         cd.put(cnt, d2, static_cast<std::uint32_t>(ref_offset(ref)));
                         ++cnt;
                     }
                 }
             }
-            // squared distances are not negative, so their bits order like the values
+#pragma unroll
+            for (int s = 0; s < 4; ++s) {
+                unsigned const m = __ballot_sync(all, leaf[s]);
+                if (leaf[s])
+                    tris[leaves + __popc(m & before)] = tri[s];
+                leaves += __popc(m);
+            }
+            // a leaf of several triangles has moved one lane's bound
             L.best = __uint_as_float(__reduce_min_sync(all, __float_as_uint(L.best)));
-            L.touched = __any_sync(all, L.touched);
+            L.touched = !(L.best > 0.0f);
+            while (leaves >= 32 && !L.touched)
+                test();
             if (L.touched)
                 break;
             cd.sort(cnt);
@@ -1023,6 +1060,8 @@ __global__ void __launch_bounds__(k_long_block) k_distance_long(spatial_params p
                 }
             sp += added;
             __syncwarp();
+            if (sp == 0 && leaves > 0)
+                test();
         }
         __syncwarp();
         if (lane == 0)
