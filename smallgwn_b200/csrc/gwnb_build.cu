@@ -526,8 +526,8 @@ __global__ void __launch_bounds__(k_block) k_collapse_level(collapse_params p, i
 // of a small one) are a chain of dependent steps, and a launch per level adds its own latency to each. A
 // barrier takes the place of the launch and a running sum that of the look-back.
 constexpr int k_narrow_block = 1024;
-// Trees of at most this many triangles are narrow throughout: 5,120 triangles, 32 launches 190 us of
-// (serialised) device time, one launch 60 us; the launches win from some 20,000 triangles on.
+// Trees of at most this many triangles are narrow throughout. Serialised device time, one launch against a
+// launch per level: 97 and 193 us at 5,120 triangles, about 185 and 190 us at 14,000, where the line lies.
 constexpr std::uint64_t k_narrow_leaves = 16384;
 // Levels of at most 4^level nodes that the top block takes (level 4 has up to 256).
 constexpr int k_narrow_top = 5;
